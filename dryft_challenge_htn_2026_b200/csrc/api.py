@@ -6,6 +6,7 @@ the sizes a kernel supports); a kernel that cannot take a size raises ``KernelEr
 compute something else. There is no CPU or library fallback behind these functions.
 """
 import ctypes
+import functools
 from ctypes import c_float, c_int, c_longlong, c_void_p
 
 import torch
@@ -134,9 +135,10 @@ class Partial:
         return self.ws.shape[1:]
 
     def sum(self, dtype=torch.bfloat16):
-        out = torch.empty(self.shape, dtype=torch.bfloat16, device=self.ws.device)
+        stored = torch.float32 if dtype == torch.float32 else torch.bfloat16
+        out = torch.empty(self.shape, dtype=stored, device=self.ws.device)
         lib = _lib("gemm.cu")
-        _check(lib, lib.dk_sum_partials(_p(self.ws), _p(out), c_longlong(out.numel()), self.ws.shape[0], _stream()),
+        _check(lib, lib.dk_sum_partials(_dt(out), _p(self.ws), _p(out), c_longlong(out.numel()), self.ws.shape[0], _stream()),
                "sum_partials")
         return out.to(dtype)
 
@@ -326,6 +328,86 @@ def sgemm(x, w, out, mode=MODE_STORE, act=(0.0, 0.0)):
         raise KernelError(f"sgemm: shapes x{tuple(x.shape)} w{tuple(w.shape)} out{tuple(out.shape)} do not match")
     lib = _lib("gemm.cu")
     _check(lib, lib.dk_sgemm(_p(x), _p(w), _p(out), M, N, K, mode, c_float(act[0]), c_float(act[1]), _stream()), "sgemm")
+
+
+# inner size from which linear() takes gemm_f32_tc: sgemm takes 0.07 us a column of K however few the rows (12 us at 64, 17 at
+# 200, 71 at 1,028, launch included), gemm_f32_tc with its split of x 17 to 25 us at all of these
+F32_TC_MIN_K = 256
+F32_CHUNK = 64              # columns of K that gemm_f32_tc adds up in tensor memory at a time
+F32_MAX_ROW_TILE = 128      # rows of x a tile
+F32_TILE_HEIGHTS = (128, 112, 96, 80, 64, 56, 48, 40, 32)      # outputs a tile (the gated product: half of them)
+
+
+def f32_groups(N, K, mode=MODE_STORE):
+    """(groups, chunks a group) of K for gemm_f32_tc: the order its sums are added up in. It depends on the weight alone,
+    never on the number of rows, so that a row's result does not depend on the rows beside it. As many groups as let
+    (128-output tile, group) units cover the SMs, of at least 8 chunks; one for the products with an activation."""
+    kb = (K + F32_CHUNK - 1) // F32_CHUNK
+    if mode in (MODE_SILU, MODE_XIELU):
+        return 1, kb
+    most = max(1, min(sm_count() // ((N + 127) // 128), kb // 8))
+    length = -(-kb // most)
+    return -(-kb // length), length
+
+
+@functools.lru_cache(maxsize=4096)
+def f32_plan(M, N, K, mode=MODE_STORE, allow_partial=False):
+    """(outputs a tile, rows of x a tile, split) for gemm_f32_tc; ``split``: a unit of work takes one group of K and leaves
+    partial sums. The plan with the least modelled time wins: waves of units x clocks of a unit. A chunk of 64 columns
+    takes the longest of its 24 mma (half a clock a row, at least 50) and its bytes (of weights at a 148th of the HBM rate, 24 a
+    clock; of weights and pieces of x at 40 a clock from the L2); a unit 2,500 more to fill and drain. Partial sums are written and read again at
+    the same rate; adding a group into ``out`` costs a unit about 1,500."""
+    sms = sm_count()
+    kb = (K + F32_CHUNK - 1) // F32_CHUNK
+    groups, length = f32_groups(N, K, mode)
+    per_out = 2 if mode == MODE_SILU else 1
+    fewest = (M + F32_MAX_ROW_TILE - 1) // F32_MAX_ROW_TILE
+    best = None
+    for row_tiles in range(fewest, fewest + 3):
+        nt = ((M + row_tiles - 1) // row_tiles + 15) // 16 * 16
+        row_tiles = (M + nt - 1) // nt
+        for height in F32_TILE_HEIGHTS:
+            tile_n = height // per_out
+            bytes_w = per_out * tile_n * 256
+            chunk = max(24 * max(nt / 2, 50), bytes_w / 24 / row_tiles, (bytes_w + 384 * nt) / 40)
+            tiles = (N + tile_n - 1) // tile_n
+            for split in ((False, True) if allow_partial and groups > 1 else (False,)):
+                units = tiles * row_tiles * (groups if split else 1)
+                unit = (length if split else kb) * chunk + 2500 + (0 if split else (groups - 1) * 1500)
+                cost = -(-units // sms) * unit + (groups * M * N * 8 / (sms * 24) if split else 0)
+                if best is None or cost < best[0]:
+                    best = cost, (tile_n, nt, split)
+    return best[1]
+
+
+def gemm_f32_tc(x, w, mode=MODE_STORE, plan=None, act=(0.0, 0.0), out=None):
+    """float32 out = x . w^T (modes and ``act`` as ``sgemm``) on tcgen05 tensor cores: both operands as three bfloat16
+    pieces, sums of 64 columns in tensor memory, everything beyond in float32 registers. K a multiple of 4, w on a 16-byte
+    boundary. A split plan gives a ``Partial``, for which K has more than one group."""
+    global _tc_err
+    _need(x, "x", torch.float32, 2), _need(w, "w", torch.float32, 2), _need(out, "out", torch.float32, 2)
+    M, K = x.shape
+    N = w.shape[0] // 2 if mode == MODE_SILU else w.shape[0]
+    tile_n, nt, split = plan or f32_plan(M, N, K, mode)
+    if K % 4 or w.shape[1] != K or w.data_ptr() % 16 or (mode == MODE_SILU and w.shape[0] % 2):
+        raise KernelError(f"gemm_f32_tc: shapes x{tuple(x.shape)} w{tuple(w.shape)} mode {mode} not supported (K % 4 == 0, aligned w)")
+    groups, length = f32_groups(N, K, mode)
+    if split and (groups == 1 or mode in (MODE_SILU, MODE_XIELU) or out is not None):
+        raise KernelError("gemm_f32_tc: nothing to split, or a result that cannot be left in parts")
+    ws = None
+    if split:
+        ws = torch.empty((groups, M, N), dtype=torch.float32, device=x.device)
+    elif out is None:
+        out = torch.empty((M, N), dtype=torch.float32, device=x.device)
+    elif tuple(out.shape) != (M, N):
+        raise KernelError(f"gemm_f32_tc: out {tuple(out.shape)} is not {(M, N)}")
+    pieces = torch.empty(3 * M * ((K + 7) // 8 * 8), dtype=torch.bfloat16, device=x.device)
+    if _tc_err is None:
+        _tc_err = torch.zeros(1, dtype=torch.int32, device=x.device)
+    lib = _lib("gemm_f32_tc.cu")
+    _check(lib, lib.dk_gemm_f32_tc(_p(x), _p(w), _p(out), _p(pieces), M, N, K, 0 if mode == MODE_STORE_F32 else mode, groups, length,
+                                   _p(ws), tile_n, nt, _p(_tc_err), c_float(act[0]), c_float(act[1]), _stream()), "gemm_f32_tc", 2)
+    return Partial(ws) if split else out
 
 
 # ---------------------------------------------------------------------------------------- sampling

@@ -123,7 +123,7 @@ def build_all(head_dims=(16, 32, 64, 128), verbose=False):
     from concurrent.futures import ThreadPoolExecutor
 
     jobs = [("elementwise.cu", None), ("attention_generic.cu", None), ("gemm.cu", None), ("gemv_stream.cu", None),
-            ("gemm_tc.cu", None), ("sampling.cu", None),
+            ("gemm_tc.cu", None), ("gemm_f32_tc.cu", None), ("sampling.cu", None),
             ("sample_noalloc.cu", None), ("attention_masked.cu", None), ("linear_attention.cu", None),
             ("short_conv.cu", None), ("moe.cu", None), ("moe_tiles.cu", None), ("latent.cu", None),
             ("group_norm.cu", None), ("recurrence.cu", None), ("stream.cu", None), ("qkv_rows.cu", None), ("delta_rule.cu", None), ("attention_talk.cu", None), ("matrix_memory.cu", None),

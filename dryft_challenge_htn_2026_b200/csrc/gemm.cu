@@ -91,18 +91,21 @@ DK_EXPORT int dk_sgemm(const float* x, const float* W, float* out, int M, int N,
 }
 
 // ----------------------------------------------------------------------------------- partial sums
-// out[m][n] = sum over slices of ws[slice][m][n], stored as bf16: for a consumer that cannot add
-// the partial sums up itself.
-__global__ void sum_partials_kernel(const float* ws, bf16* out, size_t mn, int SK) {
+// out[m][n] = sum over slices of ws[slice][m][n], stored as bf16 or float32: for a consumer that cannot
+// add the partial sums up itself.
+template <typename T>
+__global__ void sum_partials_kernel(const float* ws, T* out, size_t mn, int SK) {
     pdl_wait();
     pdl_launch_dependents();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= mn) return;
     float s = 0.f;
     for (int k = 0; k < SK; k++) s += ws[(size_t)k * mn + i];
-    out[i] = __float2bfloat16_rn(s);
+    out[i] = from_f<T>(s);
 }
 
-DK_EXPORT int dk_sum_partials(const float* ws, void* out, long long mn, int SK, cudaStream_t st) {
-    return dk_launch(sum_partials_kernel, dim3((unsigned)((mn + 255) / 256)), dim3(256), 0, st, ws, (bf16*)out, (size_t)mn, SK);
+DK_EXPORT int dk_sum_partials(int dtype, const float* ws, void* out, long long mn, int SK, cudaStream_t st) {
+    const dim3 grid((unsigned)((mn + 255) / 256));
+    if (dtype == 0) return dk_launch(sum_partials_kernel<float>, grid, dim3(256), 0, st, ws, (float*)out, (size_t)mn, SK);
+    return dk_launch(sum_partials_kernel<bf16>, grid, dim3(256), 0, st, ws, (bf16*)out, (size_t)mn, SK);
 }

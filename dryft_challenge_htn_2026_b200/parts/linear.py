@@ -1,6 +1,8 @@
 """out = x . W^T for a weight [out, in] without bias: picks the kernel by dtype and row count.
 
-float32: the CUDA-core sgemm for every size (a true 32-bit product). bfloat16: up to 8 rows the
+float32: the tensor-core product of three bfloat16 pieces (24 significant bits; gemm_f32_tc.cu) from an inner size of
+256 on, the CUDA-core sgemm below and where rows do not sit on 16-byte boundaries; which of the two depends on the weight
+alone, so a row's result never depends on the rows beside it. bfloat16: up to 8 rows the
 streaming kernel (cp.async rings, weights read once); up to 128 rows the TMA + tcgen05 kernel in its
 decode form (one tile of rows, K in slices); for more rows (prefill) the same kernel, always for the
 gated product (SiLU*up fused into its epilogue) and otherwise when its 128 x 256 tiles fill the
@@ -24,6 +26,9 @@ def linear(x, w, mode=STORE, allow_partial=False, act=(0.0, 0.0)):
     M, K = x.shape
     N = w.shape[0] // 2 if mode == SILU else w.shape[0]
     if x.dtype == torch.float32:
+        if K >= api.F32_TC_MIN_K and K % 4 == 0 and w.data_ptr() % 16 == 0:
+            plan = api.f32_plan(M, N, K, mode, allow_partial)
+            return api.gemm_f32_tc(x, w, mode, plan, act)
         out = torch.empty((M, N), dtype=torch.float32, device=x.device)
         api.sgemm(x, w, out, mode, act)
         return out

@@ -1,0 +1,79 @@
+"""The float32 tensor-core product (gemm_f32_tc) against float64, at the edges of its tiles, chunks and groups."""
+import pytest
+import torch
+
+from dryft_challenge_htn_2026_b200.csrc import api
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def rnd(*shape, seed, scale=1.0):
+    g = torch.Generator().manual_seed(seed)
+    return (torch.randn(*shape, generator=g) * scale).to(DEV)
+
+
+def bound(x, w):
+    """|error| of a sum of K terms: the pieces leave out 2^-24 of |x||w|; a chunk adds at most 8 times to a 24-bit sum that may be cut
+    off (2^-23), the chunks and groups at most K / 64 + 2 times in float32 (2^-24). Each relative to sum |x w|."""
+    K = x.shape[1]
+    return (2.0 ** -24 + 8 * 2.0 ** -23 + (K // 64 + 3) * 2.0 ** -24) * (x.double().abs() @ w.double().abs().T) + 1e-30
+
+
+@pytest.mark.parametrize("N,K", [(1, 4), (64, 64), (129, 68), (257, 1028), (130, 4096), (20000, 260)])
+@pytest.mark.parametrize("M", [1, 16, 17, 129])
+def test_plain_product(M, N, K):
+    x, w = rnd(M, K, seed=1), rnd(N, K, seed=2)
+    ref = x.double() @ w.double().T
+    out = api.gemm_f32_tc(x, w)
+    assert bool(((out.double() - ref).abs() <= bound(x, w)).all())
+    # the same sums in the same order, whatever the tiles, the split and the rows beside
+    for plan in [(32, 16, False), (128, 128, False)] + ([(128, 48, True)] if api.f32_groups(N, K)[0] > 1 else []):
+        again = api.gemm_f32_tc(x, w, plan=plan)
+        again = again.sum(torch.float32) if isinstance(again, api.Partial) else again
+        assert torch.equal(again, out), plan
+    assert torch.equal(api.gemm_f32_tc(x[M // 2:M // 2 + 1].clone(), w)[0], out[M // 2])
+    api.gemm_tc_check()
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 65, 72), (40, 200, 260), (130, 64, 128)])
+def test_activations(M, N, K):
+    x, w = rnd(M, K, seed=3), rnd(2 * N, K, seed=4, scale=0.3)
+    y, slack = x.double() @ w.double().T, bound(x, w)
+    g, u = y[:, :N], y[:, N:]
+    out = torch.empty(M, N, device=DEV)
+    for act in ((0.0, 0.0), api.GATE_GELU, api.gate_clamped(1.5)):
+        got = api.gemm_f32_tc(x, w, api.MODE_SILU, act=act)
+        api.sgemm(x, w, out, api.MODE_SILU, act)
+        # slopes of the gates are at most 1.2 in g; sgemm's own sums are off by K roundings
+        far = (1 + K / 16) * 1.2 * (slack[:, :N] * (u.abs() + 1) + slack[:, N:] * (g.abs() + 1)) + 1e-6
+        assert bool(((got - out).abs() <= far).all()), act
+    z = y[:, :N]
+    got = api.gemm_f32_tc(x, w[:N].contiguous(), api.MODE_XIELU, act=(0.7, 0.3))
+    ref = torch.where(z > 0, 0.7 * z * z, 0.3 * (torch.expm1(z) - z)) + 0.5 * z
+    assert bool(((got.double() - ref).abs() <= slack[:, :N] * (1.4 * z.abs() + 1) + 1e-6).all())
+
+
+def test_values_that_are_not_finite():
+    """An infinity, a NaN and a number that rounds to infinity in bfloat16 give what the FMA product gives, and only there."""
+    x, w = rnd(5, 300, seed=5), rnd(200, 300, seed=6)
+    clean = api.gemm_f32_tc(x, w)
+    x[1, 3], x[2, 7], w[9, 4], x[3, 9] = float("inf"), float("nan"), float("-inf"), 3.4e38
+    got, ref = api.gemm_f32_tc(x, w), torch.empty(5, 200, device=DEV)
+    api.sgemm(x, w, ref)
+    assert torch.equal(got.isnan(), ref.isnan()) and torch.equal(got.isinf(), ref.isinf())
+    assert torch.equal(got[got.isinf()], ref[ref.isinf()])
+    assert torch.allclose(got[3][ref[3].isfinite()], ref[3][ref[3].isfinite()], rtol=1e-5)
+    keep = torch.ones(200, dtype=torch.bool, device=DEV)
+    keep[9] = False
+    assert torch.equal(got[[0, 4]][:, keep], clean[[0, 4]][:, keep])
+
+
+def test_refusals():
+    x, w = rnd(2, 64, seed=7), rnd(8, 64, seed=8)
+    with pytest.raises(api.KernelError):
+        api.gemm_f32_tc(x[:, :62].contiguous(), w[:, :62].contiguous())
+    with pytest.raises(api.KernelError):
+        api.gemm_f32_tc(x, rnd(8 * 64 + 1, seed=9)[1:].view(8, 64))
+    with pytest.raises(api.KernelError):
+        api.gemm_f32_tc(x, w, plan=(32, 16, True))
