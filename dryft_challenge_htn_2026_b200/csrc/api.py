@@ -232,6 +232,43 @@ def attention_generic(q, out, k_store, v_store, row_pos, row_seq, page_table, n_
                                          head_dim, int(window or 0), c_float(scale), _stream()), "attention_generic")
 
 
+F32_ATTENTION_HEAD_DIMS = (64, 128)
+F32_ATTENTION_MAX_GROUP = 16        # query heads a kv head
+F32_TILE_ROWS = 64                  # rows (queries x the query heads of a kv head) a block of attention_prompt_f32 takes
+
+
+def _need_f32_attention(q, out, k_store, v_store, page_table, n_heads, n_kv_heads, head_dim):
+    _need(q, "q", torch.float32, 2), _need(out, "out", torch.float32, 2), _need(page_table, "page_table", torch.int32, 2)
+    _need(k_store, "k_store", torch.float32), _need(v_store, "v_store", torch.float32)
+    if head_dim not in F32_ATTENTION_HEAD_DIMS or n_heads % n_kv_heads or n_heads // n_kv_heads > F32_ATTENTION_MAX_GROUP \
+            or q.shape[1] != n_heads * head_dim or out.shape != q.shape:
+        raise KernelError(f"float32 attention: head size {head_dim} (64 or 128) / heads {n_heads}:{n_kv_heads} not supported")
+
+
+def attention_prompt_f32(q, out, k_store, v_store, tiles, cu_q, seq_pos0, page_table, n_heads, n_kv_heads, head_dim, window, scale):
+    """Float32 attention of portions of prompts (head sizes 64 and 128). ``tiles`` lists tiles of F32_TILE_ROWS // (query heads a kv
+    head) queries as for ``attention_prefill_bf16``. A row gives the bits ``attention_decode_f32`` gives for it."""
+    _need_f32_attention(q, out, k_store, v_store, page_table, n_heads, n_kv_heads, head_dim)
+    _need(tiles, "tiles", torch.int32, 2), _need(cu_q, "cu_q", torch.int32, 1), _need(seq_pos0, "seq_pos0", torch.int32, 1)
+    lib = _lib("attention_f32.cu", {"HD": head_dim})
+    _check(lib, lib.dk_attn_f32_prompt(_p(q), _p(out), _p(k_store), _p(v_store), _p(tiles), tiles.shape[0], _p(cu_q), _p(seq_pos0),
+                                       _p(page_table), page_table.shape[1], n_heads, n_kv_heads, int(window or 0), c_float(scale),
+                                       _stream()), "attention_prompt_f32")
+
+
+def attention_decode_f32(q, out, k_store, v_store, row_pos, page_table, n_heads, n_kv_heads, head_dim, window, scale):
+    """Float32 attention of one token a sequence (head sizes 64 and 128): a block a page of keys, merged in order by a second kernel."""
+    _need_f32_attention(q, out, k_store, v_store, page_table, n_heads, n_kv_heads, head_dim)
+    _need(row_pos, "row_pos", torch.int32, 1)
+    n_seq, pages = q.shape[0], page_table.shape[1]
+    ws = torch.empty(n_seq * n_heads * pages * (head_dim + 2), dtype=torch.float32, device=q.device)
+    cut = n_seq * n_heads * pages * head_dim
+    lib = _lib("attention_f32.cu", {"HD": head_dim})
+    _check(lib, lib.dk_attn_f32_decode(_p(q), _p(out), _p(k_store), _p(v_store), _p(row_pos), _p(page_table), pages, n_seq, n_heads,
+                                       n_kv_heads, int(window or 0), c_float(scale), _p(ws), _p(ws[cut:]), _stream()),
+           "attention_decode_f32", 2)
+
+
 def _attn_lib(head_dim):
     if head_dim % 16 or not 16 <= head_dim <= 256:
         raise KernelError(f"bfloat16 attention: head size {head_dim} not supported (multiples of 16 up to 256)")

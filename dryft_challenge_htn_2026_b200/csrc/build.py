@@ -130,6 +130,7 @@ def build_all(head_dims=(16, 32, 64, 128), verbose=False):
             ("attention_shared_rows.cu", {"HD": 576, "HDV": 512})]
     jobs += [("attention_bf16.cu", {"HD": hd}) for hd in head_dims]
     jobs += [("attention_tc.cu", {"HD": hd}) for hd in head_dims if hd in (64, 128)]
+    jobs += [("attention_f32.cu", {"HD": hd}) for hd in head_dims if hd in (64, 128)]
     jobs += [("attention_tc.cu", {"HD": hd, "DK_MASKED": 1}) for hd in head_dims if hd in (64, 128)]
     jobs += [("attention_bf16.cu", {"HD": hd, "DK_MASKED": 1}) for hd in head_dims if hd in (64, 128)]
     jobs += [("attention_masked_bf16.cu", {"HD": hd, "HDV": hd}) for hd in head_dims if hd in (64, 128)]

@@ -61,8 +61,13 @@ class GQAAttention(Part):
         self.max_positions = 0
         # the prefill kernel this mixer's steps use, and so the tiles they need planned
         self.tc_prefill = rt.dtype == torch.bfloat16 and s.head_dim in api.TC_ATTENTION_HEAD_DIMS
+        # float32: tiles of rows and a block a page where the kernels take the head size, a warp a row elsewhere. The heads alone
+        # decide, so that a row's result does not depend on what it is computed with.
+        group = s.num_heads // s.num_kv_heads
+        self.paged_f32 = rt.dtype == torch.float32 and s.head_dim in api.F32_ATTENTION_HEAD_DIMS \
+            and group <= api.F32_ATTENTION_MAX_GROUP
         self.tiles = QueryTiles(api.TC_TILE_ROWS if self.tc_prefill else api.MMA_TILE_ROWS) \
-            if rt.dtype == torch.bfloat16 else None
+            if rt.dtype == torch.bfloat16 else QueryTiles(api.F32_TILE_ROWS // group) if self.paged_f32 else None
 
     def param_decls(self):
         s = self.spec
@@ -145,7 +150,12 @@ class GQAAttention(Part):
         nh, nkv, hd = s.num_heads, s.num_kv_heads, s.head_dim
         window = s.window or 0
         o = torch.empty((ctx.n_tok, nh * hd), dtype=dtype, device=dev)
-        if dtype == torch.float32:
+        if self.paged_f32 and ctx.is_decode:
+            api.attention_decode_f32(q, o, kv.k, kv.v, ctx.row_pos, table, nh, nkv, hd, window, s.scale)
+        elif self.paged_f32:
+            api.attention_prompt_f32(q, o, kv.k, kv.v, ctx.plans[self.tiles.key], ctx.cu_q, ctx.seq_pos0, table, nh, nkv, hd, window,
+                                     s.scale)
+        elif dtype == torch.float32:
             api.attention_generic(q, o, kv.k, kv.v, ctx.row_pos, ctx.row_seq, table, nh, nkv, hd, window, s.scale)
         elif ctx.is_decode:
             nsplit = api.decode_splits(ctx.n_seq, nkv, nh // nkv, table.shape[1])

@@ -1,0 +1,58 @@
+"""Float32 attention of prompts and of single tokens over the paged cache against float64: ragged portions, pages that end inside a
+tile, windows, groups that do not divide a tile, and bits that do not depend on which of the two kernels a token goes through."""
+import numpy as np
+import pytest
+import torch
+
+from dryft_challenge_htn_2026_b200.csrc import api
+from dryft_challenge_htn_2026_b200.parts.attention import QueryTiles
+from test_kernels_gpu import paged_setup, rnd
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def ref64(q, s, nh, nkv, hd, window):
+    out = torch.empty(q.shape[0], nh, hd, dtype=torch.float64, device=DEV)
+    qd = q.double().view(-1, nh, hd)
+    for t in range(q.shape[0]):
+        i, p = int(s["row_seq"][t]), int(s["row_pos"][t])
+        lo = max(0, p - window + 1) if window else 0
+        K, V = (s[x][i][lo:p + 1].double().repeat_interleave(nh // nkv, 1) for x in ("dense_k", "dense_v"))
+        w = torch.softmax(torch.einsum("phd,hd->hp", K, qd[t]) * hd ** -0.5, -1)
+        out[t] = torch.einsum("hp,phd->hd", w, V)
+    return out.view(q.shape[0], nh * hd)
+
+
+@pytest.mark.parametrize("nh,nkv,hd,window", [(8, 2, 128, 0), (4, 4, 64, 0), (6, 2, 128, 90), (16, 1, 64, 7), (10, 2, 64, 64)])
+def test_attention_f32(nh, nkv, hd, window):
+    before, new = [0, 100, 0, 63, 130, 640], [70, 150, 1, 2, 65, 17]
+    s = paged_setup(before, new, nkv, hd, torch.float32, seed=5)
+    s["k_store"].masked_fill_(s["k_store"] == 0, float("nan"))      # what no token wrote must not reach any result
+    s["v_store"].masked_fill_(s["v_store"] == 0, float("nan"))
+    q = rnd(s["n_tok"], nh * hd, seed=6)
+    plan = QueryTiles(api.F32_TILE_ROWS // (nh // nkv)).build(new, before, False)
+    out = torch.full_like(q, float("nan"))
+    api.attention_prompt_f32(q, out, s["k_store"], s["v_store"], torch.tensor(plan, device=DEV), s["cu_q"], s["pos0"], s["table"], nh,
+                             nkv, hd, window, hd ** -0.5)
+    ref = ref64(q, s, nh, nkv, hd, window)
+    # scores of unit normal heads: below 8 with hd / 4 roundings of 2^-24 of their terms each, as an error of the weights; the
+    # values' sum adds 64 + pages more: 2e-5 of the largest value (4.5) bounds both
+    assert float((out.double() - ref).abs().max()) <= 2e-5 * 4.5
+    # the same tokens one by one, the sequences in another order and a padding row among them
+    rows = torch.tensor([0, 69, 70, 219, 220, 221, 222, 230, 287, s["n_tok"] - 1], device=DEV)
+    pos, seq = s["row_pos"][rows].clone(), s["row_seq"][rows].long()
+    pos[4] = -1
+    one = torch.full((len(rows), nh * hd), float("nan"), device=DEV)
+    api.attention_decode_f32(q[rows].contiguous(), one, s["k_store"], s["v_store"], pos, s["table"][seq].contiguous(), nh, nkv, hd,
+                             window, hd ** -0.5)
+    assert float(one[4].abs().max()) == 0.0
+    keep = np.array([i for i in range(len(rows)) if i != 4])
+    assert torch.equal(one[keep], out[rows][keep])
+
+
+def test_refusals():
+    s = paged_setup([0], [3], 1, 32, torch.float32, seed=7)
+    q = rnd(3, 64, seed=8)
+    with pytest.raises(api.KernelError):
+        api.attention_decode_f32(q, torch.empty_like(q), s["k_store"], s["v_store"], s["row_pos"], s["table"], 2, 1, 32, 0, 0.1)
