@@ -20,7 +20,11 @@ class KernelError(RuntimeError):
     pass
 
 
-_pdl = False
+# On from the start: a decode step is a chain of kernels of 2 to 20 us whose starts and first loads then lie under the end of the
+# kernel before (Qwen3-4B sizes, generation as a whole: one sequence 84.0 -> 69.6 ms, 16 sequences 458 -> 399, a first step of 9
+# tokens 2.90 -> 2.61). Kernels of many rows are launched without (dk_launch_whole): with it a prompt of 2,048 tokens took 16.36 ms
+# instead of 16.13.
+_pdl = True
 
 
 def set_pdl(on):

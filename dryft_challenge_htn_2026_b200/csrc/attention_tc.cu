@@ -694,7 +694,7 @@ DK_EXPORT int dk_attn_prefill_tc(const void* q, void* out, const void* k_store, 
     if (n_items > 0x7fffffffLL - 4 * sms) return (int)cudaErrorInvalidValue;
     const long long slots = (long long)BLOCKS_PER_SM * sms;
     const int blocks = (int)(n_items < slots ? n_items : slots);
-    return dk_launch(attn_prefill_tc_kernel, dim3(blocks), dim3(THREADS), smem, st, mq, mk, mv, (bf16*)out, tiles, (int)n_items,
+    return dk_launch_whole(attn_prefill_tc_kernel, dim3(blocks), dim3(THREADS), smem, st, mq, mk, mv, (bf16*)out, tiles, (int)n_items,
                      cu_q, seq_pos0, page_table, pt_stride, nh, nkv, window, scale * 1.4426950408889634f, err, sched);
 }
 #else
@@ -728,7 +728,7 @@ DK_EXPORT int dk_attn_prefill_tc_masked(const void* q, long long ldq, void* out,
     if (n_items > 0x7fffffffLL - 4 * sms) return (int)cudaErrorInvalidValue;
     const long long slots = (long long)BLOCKS_PER_SM * sms;
     const int blocks = (int)(n_items < slots ? n_items : slots);
-    return dk_launch(attn_prefill_tc_kernel, dim3(blocks), dim3(THREADS), smem, st, mq, mk, mv, (bf16*)out, tiles, (int)n_items,
+    return dk_launch_whole(attn_prefill_tc_kernel, dim3(blocks), dim3(THREADS), smem, st, mq, mk, mv, (bf16*)out, tiles, (int)n_items,
                      cu_q, seq_pos0, page_table, pt_stride, nh, nkv, window, scale * 1.4426950408889634f, err, sched, ldo,
                      (const bf16*)gate, ldg, out_scale, chunk, keep_first, softcap > 0.f ? softcap * 1.4426950408889634f : 0.f,
                      softcap > 0.f ? scale / softcap : 0.f, r1, r2, sink);

@@ -514,13 +514,13 @@ DK_EXPORT int dk_add_rmsnorm(int dtype, float* h, const void* delta, const float
         const dim3 grid((n_rows + wpb - 1) / wpb), block(32 * wpb);
 #define NORM_WARP(CH)                                                                                                   \
     if (H == CH * 256)                                                                                                  \
-        return dk_launch(add_rmsnorm_warp_kernel<CH>, grid, block, 0, st, h, (const bf16*)delta, w, eps, n_rows, (bf16*)a)
+        return dk_launch_whole(add_rmsnorm_warp_kernel<CH>, grid, block, 0, st, h, (const bf16*)delta, w, eps, n_rows, (bf16*)a)
         NORM_WARP(1); NORM_WARP(2); NORM_WARP(3); NORM_WARP(4); NORM_WARP(5); NORM_WARP(6); NORM_WARP(7); NORM_WARP(8);
         NORM_WARP(9); NORM_WARP(10); NORM_WARP(11); NORM_WARP(12); NORM_WARP(13); NORM_WARP(14); NORM_WARP(15); NORM_WARP(16);
 #undef NORM_WARP
     }
     if (dtype == 1 && parts == nullptr && rows == nullptr && H % 8 == 0 && H <= 8 * 4 * row_threads(H) && n_rows > 64)
-        return dk_launch(add_rmsnorm_wide_kernel, dim3(n_rows), dim3(row_threads(H)), 0, st, h, (const bf16*)delta, w, eps,
+        return dk_launch_whole(add_rmsnorm_wide_kernel, dim3(n_rows), dim3(row_threads(H)), 0, st, h, (const bf16*)delta, w, eps,
                          H, (bf16*)a);
     if ((n_rows <= 64 || parts != nullptr) && H % 4 == 0 && H <= 8192 && part_stride % 4 == 0) {
         if (H <= 4096) {
@@ -561,7 +561,7 @@ DK_EXPORT int dk_qk_norm_rope_write(int dtype, const void* qkv, const float* par
         const int gs = half8 <= 1 ? 1 : half8 <= 2 ? 2 : half8 <= 4 ? 4 : half8 <= 8 ? 8 : 16;
         const unsigned wblocks = (unsigned)((warps + 4LL * (32 / gs) - 1) / (4LL * (32 / gs)));
 #define ROPE_WIDE(GS)                                                                                                  \
-    return dk_launch(qk_norm_rope_write_wide_kernel<GS>, dim3(wblocks), dim3(128), 0, st, (const bf16*)qkv, (bf16*)q_out, \
+    return dk_launch_whole(qk_norm_rope_write_wide_kernel<GS>, dim3(wblocks), dim3(128), 0, st, (const bf16*)qkv, (bf16*)q_out, \
                      (bf16*)dense_out, qn, kn, cos_t, sin_t, row_pos, row_seq, page_table, pt_stride, (bf16*)k_store, (bf16*)v_store, n_tok, \
                      nh, nkv, hd, eps, write_kv)
         if (gs == 1) ROPE_WIDE(1);
