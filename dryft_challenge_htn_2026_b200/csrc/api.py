@@ -531,6 +531,24 @@ def stream_plan(M, N, K, mode, allow_partial=False):
     return sk, blocks, warps
 
 
+STREAM_SMALL_WEIGHTS = 8 << 20              # numbers of a matrix below which few rows always take the streaming product
+
+
+def few_rows_stream_plan(M, N, K, mode, allow_partial=False):
+    """The streaming product's plan for up to STREAM_BEST_ROWS rows, or None where the tensor-core product in its decode form
+    (``skinny_tc_plan``) is the faster one: products that may stay in parts and are at least as deep as wide (a layer's output
+    and down projections). While whole rows of x fit they stream in one slice with eight warps a block, since every slice costs the
+    norm behind it (2,560 outputs of 4,096 at 8 rows, in a chain norm - product: 8.7 us, 9.4 in four slices as two blocks an SM,
+    9.6 on the tensor cores; 4,096 of 4,096: 10.2, 11.0, 10.9); deeper ones go to the tensor cores (2,560 of 9,728: 14.9 -> 13.9;
+    4,096 of 12,288: 24.0 -> 22.2; 5,120 of 17,408: 39.0 -> 35.1). Generation with both: one sequence of 4B sizes 69.2 -> 67.9 ms,
+    eight 252 -> 244, three of 8B sizes 98.2 -> 95.4. The gated and the q/k/v product are as fast or faster there alone (21.2 against 22.3
+    us, 8.9 against 9.1), but whole generations were 1 to 4 % slower with them on the tensor cores: their blocks take an SM's whole
+    shared memory, which the attention and rotation between them then wait for. Small matrices stay with ``stream_plan``."""
+    if allow_partial and mode in (MODE_STORE, MODE_STORE_F32) and N <= K and N * K >= STREAM_SMALL_WEIGHTS:
+        return (1, sm_count(), 8) if _stream_smem(M, K, 1, 8) <= _STREAM_SMEM_BLOCK else None
+    return stream_plan(M, N, K, mode, allow_partial)
+
+
 def gemv_stream(x, w, out=None, mode=MODE_STORE, plan=None, act=(0.0, 0.0)):
     """The weight-streaming skinny product (asynchronous copies into shared-memory rings,
     tensor-core multiply) for at most 16 rows of x and K a multiple of 16. Returns ``out`` [M, N]
@@ -666,6 +684,10 @@ def skinny_tc_plan(M, N, K, mode, allow_partial=False):
         return min(TC_TILE_HEIGHTS, key=lambda bn: (bn * -(-((N + bn - 1) // bn) // sms), bn)), 1
     if mode != MODE_STORE or not allow_partial:
         return 256, 1
+    if M <= 32:
+        plan = _few_units_plan(N, kb, sms)
+        if plan is not None:
+            return plan
     plans = []
     for bn in TC_TILE_HEIGHTS:
         tiles = (N + bn - 1) // bn
@@ -677,6 +699,29 @@ def skinny_tc_plan(M, N, K, mode, allow_partial=False):
     least = min(p[0] for p in plans)
     _, sk, bn = min((p for p in plans if p[0] <= 1.03 * least), key=lambda p: (p[1], p[0], -p[2]))
     return bn, sk
+
+
+def _few_units_plan(N, kb, sms):
+    """skinny_tc_plan up to 32 rows: units for at most nine tenths of the SMs, the tallest tiles among equals. From about 136
+    units of 148 on the chain norm - product - norm takes 1 to 2 us longer (16 rows, 4,096 outputs of 4,096: 145 units 14.1 us, 130
+    units of the same length 12.4), since the short kernels around it find no SM of their own; and a block of K costs a unit
+    about as much as 40 more weight rows, a slice as much as 50 rows. Against the smallest unit on all SMs (us at 16 rows): 6,144
+    outputs of 2,560 10.8 -> 9.6, 2,560 of 4,096 11.0 -> 10.1, 2,560 of 9,728 16.0 -> 14.4; 6,144 of 4,096 15.1 -> 13.1, 4,096 of
+    4,096 14.1 -> 12.0, 4,096 of 12,288 24.9 -> 23.0; 7,168 of 5,120 18.2 -> 17.0, 5,120 of 5,120 18.0 -> 16.3, 5,120 of 17,408
+    37.3 -> 35.8. At 64 rows it is the other way round (2,560 of 9,728 16.4 -> 16.7). Whole generations of 16 sequences: 397 -> 391
+    ms, a first step of 9 tokens 2.60 -> 2.55. None: the tiles alone are too many."""
+    room = sms * 9 // 10 - 1
+    best = None
+    for bn in TC_TILE_HEIGHTS:
+        tiles = (N + bn - 1) // bn
+        for sk in range(1, room // tiles + 1):
+            length = (kb + sk - 1) // sk
+            if sk > 1 and ((sk - 1) * length >= kb or length < 6):
+                continue
+            cost = length * (bn + 40) + 50 * sk
+            if best is None or cost < best[0]:
+                best = cost, (bn, sk)
+    return best and best[1]
 
 
 def gated_tc_plan(M, N):

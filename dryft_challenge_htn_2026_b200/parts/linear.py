@@ -3,8 +3,8 @@
 float32: the tensor-core product of three bfloat16 pieces (24 significant bits; gemm_f32_tc.cu) from an inner size of
 256 on, the CUDA-core sgemm below and where rows do not sit on 16-byte boundaries; which of the two depends on the weight
 alone, so a row's result never depends on the rows beside it. bfloat16: up to 8 rows the
-streaming kernel (cp.async rings, weights read once); up to 128 rows the TMA + tcgen05 kernel in its
-decode form (one tile of rows, K in slices); for more rows (prefill) the same kernel, always for the
+streaming kernel (cp.async rings, weights read once) where it is the faster one (``csrc.api.few_rows_stream_plan``); up to
+128 rows the TMA + tcgen05 kernel in its decode form (one tile of rows, K in slices); for more rows (prefill) the same kernel, always for the
 gated product (SiLU*up fused into its epilogue) and otherwise when its 128 x 256 tiles fill the
 GPU's waves, else the library matrix product (the reference uses the library for all of these,
 engine/fused.py:993-995)."""
@@ -51,7 +51,7 @@ def linear(x, w, mode=STORE, allow_partial=False, act=(0.0, 0.0)):
             api.xielu(out, out, act[0], act[1])
         return out
     if M <= api.STREAM_BEST_ROWS and K % 16 == 0:
-        plan = api.stream_plan(M, N, K, mode, allow_partial)
+        plan = api.few_rows_stream_plan(M, N, K, mode, allow_partial)
         if plan is not None:
             return api.gemv_stream(x, w, None, mode, plan, act)
     if M <= api.TC_SKINNY_MAX_ROWS:
