@@ -540,12 +540,16 @@ def few_rows_stream_plan(M, N, K, mode, allow_partial=False):
     and down projections). While whole rows of x fit they stream in one slice with eight warps a block, since every slice costs the
     norm behind it (2,560 outputs of 4,096 at 8 rows, in a chain norm - product: 8.7 us, 9.4 in four slices as two blocks an SM,
     9.6 on the tensor cores; 4,096 of 4,096: 10.2, 11.0, 10.9); deeper ones go to the tensor cores (2,560 of 9,728: 14.9 -> 13.9;
-    4,096 of 12,288: 24.0 -> 22.2; 5,120 of 17,408: 39.0 -> 35.1). Generation with both: one sequence of 4B sizes 69.2 -> 67.9 ms,
-    eight 252 -> 244, three of 8B sizes 98.2 -> 95.4. The gated and the q/k/v product are as fast or faster there alone (21.2 against 22.3
+    4,096 of 12,288: 24.0 -> 22.2; 5,120 of 17,408: 39.0 -> 35.1). Generation with both: one sequence of 4B sizes 69.2 -> 67.0 ms,
+    eight 252 -> 242, three of 8B sizes 98.2 -> 96.0. The gated and the q/k/v product are as fast or faster there alone (21.2 against 22.3
     us, 8.9 against 9.1), but whole generations were 1 to 4 % slower with them on the tensor cores: their blocks take an SM's whole
-    shared memory, which the attention and rotation between them then wait for. Small matrices stay with ``stream_plan``."""
+    shared memory, which the attention and rotation between them then wait for. Small matrices stay with ``stream_plan``. Sums that
+    left in parts, in float32, still do: one slice is one part (``linear``)."""
     if allow_partial and mode in (MODE_STORE, MODE_STORE_F32) and N <= K and N * K >= STREAM_SMALL_WEIGHTS:
-        return (1, sm_count(), 8) if _stream_smem(M, K, 1, 8) <= _STREAM_SMEM_BLOCK else None
+        if _stream_smem(M, K, 1, 8) <= _STREAM_SMEM_BLOCK:
+            return 1, sm_count(), 8
+        if skinny_tc_plan(M, N, K, MODE_STORE, True)[1] > 1:
+            return None
     return stream_plan(M, N, K, mode, allow_partial)
 
 
@@ -709,14 +713,15 @@ def _few_units_plan(N, kb, sms):
     outputs of 2,560 10.8 -> 9.6, 2,560 of 4,096 11.0 -> 10.1, 2,560 of 9,728 16.0 -> 14.4; 6,144 of 4,096 15.1 -> 13.1, 4,096 of
     4,096 14.1 -> 12.0, 4,096 of 12,288 24.9 -> 23.0; 7,168 of 5,120 18.2 -> 17.0, 5,120 of 5,120 18.0 -> 16.3, 5,120 of 17,408
     37.3 -> 35.8. At 64 rows it is the other way round (2,560 of 9,728 16.4 -> 16.7). Whole generations of 16 sequences: 397 -> 391
-    ms, a first step of 9 tokens 2.60 -> 2.55. None: the tiles alone are too many."""
+    ms, a first step of 9 tokens 2.60 -> 2.55. None: no room for two slices (one
+    would leave as bfloat16 where the caller had float32 parts)."""
     room = sms * 9 // 10 - 1
     best = None
     for bn in TC_TILE_HEIGHTS:
         tiles = (N + bn - 1) // bn
-        for sk in range(1, room // tiles + 1):
+        for sk in range(2, room // tiles + 1):
             length = (kb + sk - 1) // sk
-            if sk > 1 and ((sk - 1) * length >= kb or length < 6):
+            if (sk - 1) * length >= kb or length < 6:
                 continue
             cost = length * (bn + 40) + 50 * sk
             if best is None or cost < best[0]:

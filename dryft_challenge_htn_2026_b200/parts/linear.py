@@ -52,6 +52,9 @@ def linear(x, w, mode=STORE, allow_partial=False, act=(0.0, 0.0)):
         return out
     if M <= api.STREAM_BEST_ROWS and K % 16 == 0:
         plan = api.few_rows_stream_plan(M, N, K, mode, allow_partial)
+        if plan is not None and plan[0] == 1 and mode == STORE and plan != api.stream_plan(M, N, K, mode, allow_partial):
+            # one slice where there were several: its float32 sums go on as the only part, not rounded in between
+            return api.Partial(api.gemv_stream(x, w, None, STORE_F32, plan, act).unsqueeze(0))
         if plan is not None:
             return api.gemv_stream(x, w, None, mode, plan, act)
     if M <= api.TC_SKINNY_MAX_ROWS:

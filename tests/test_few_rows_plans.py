@@ -30,6 +30,8 @@ def test_units_of_up_to_32_rows_leave_sms_to_the_kernels_around_them():
         kb, tiles = (K + 63) // 64, (N + bn - 1) // bn
         assert bn in api.TC_TILE_HEIGHTS and sk >= 1 and (sk == 1 or (sk - 1) * ((kb + sk - 1) // sk) < kb)
         assert tiles * sk < 0.9 * sms or N == 33000
+        if (N + 255) // 256 <= sms // 4 and K >= 2560:
+            assert sk > 1                                 # float32 parts, as many rows as few
     if sms == 148:
         assert api.skinny_tc_plan(16, 2560, 4096, api.MODE_STORE, True) == (160, 8)
         assert api.skinny_tc_plan(16, 4096, 12288, api.MODE_STORE, True) == (256, 8)
