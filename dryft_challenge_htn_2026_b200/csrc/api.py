@@ -7,6 +7,7 @@ compute something else. There is no CPU or library fallback behind these functio
 """
 import ctypes
 import functools
+import threading
 from ctypes import c_float, c_int, c_longlong, c_void_p
 
 import torch
@@ -20,19 +21,50 @@ class KernelError(RuntimeError):
     pass
 
 
-# On from the start: a decode step is a chain of kernels of 2 to 20 us whose starts and first loads then lie under the end of the
-# kernel before (Qwen3-4B sizes, generation as a whole: one sequence 84.0 -> 69.6 ms, 16 sequences 458 -> 399, a first step of 9
-# tokens 2.90 -> 2.61). Kernels of many rows are launched without (dk_launch_whole): with it a prompt of 2,048 tokens took 16.36 ms
-# instead of 16.13.
-_pdl = True
+# Dependent launches (a kernel starts, and asks for what no kernel of a step writes, under the end of the kernel before): None
+# for the rule below, or what set_pdl() chose for every launch.
+_pdl = None
+
+
+class _Thread(threading.local):
+    """What one thread's launches are: inside a model's step or not, and what each library was last told."""
+    steps = 0            # model steps this thread is in the middle of
+    dependent = False    # whether the next launch is a dependent one
+
+    def __init__(self):
+        self.told = {}
+
+
+_thread = _Thread()
+
+
+class dependent_launches:
+    """``with dependent_launches():`` around the kernels of a model's step. Kernels launched here start under the end of the one
+    before them, and some of them read before they wait for it: matrix products their weights, the norms and rotations their
+    weights, positions and tables, decode attention its positions, page ids and the cache pages before the newest token's. So
+    nothing launched in here may write any of those. The first launch waits for all that the stream held before, so that the
+    caller may have. Outside, where any call may read what the one before it wrote, every kernel is launched behind the full
+    end of the one before. It holds for the calling thread only.
+
+    A decode step is a chain of kernels of 2 to 20 us, and pays for every gap between them without. Kernels of a Qwen3 prompt gain
+    nothing and are launched whole here too (dk_launch_whole)."""
+
+    def __enter__(self):
+        _thread.steps += 1
+
+    def __exit__(self, *exc):
+        _thread.steps -= 1
+        if _thread.steps == 0:
+            _thread.dependent = False
 
 
 def set_pdl(on):
-    """Programmatic dependent launch for every kernel launched from here on."""
+    """Programmatic dependent launch for every kernel launched from here on (on or off), in a model's step or not; None: in the
+    steps alone, as it is from the start. With it on, a caller of single functions keeps to the rule of ``dependent_launches``."""
     global _pdl
-    _pdl = bool(on)
+    _pdl = None if on is None else bool(on)
     for lib in list(build._libs.values()):
-        lib.dk_set_pdl(int(_pdl))
+        lib.dk_set_pdl(int(bool(_pdl)))
 
 
 _cuda_seen = False
@@ -48,9 +80,14 @@ def _lib(source, defines=None):
     fresh = key not in build._libs
     lib = build.load_lib(source, defines)
     if fresh:
-        lib.dk_set_pdl.argtypes = [c_int]
-        lib.dk_set_pdl(int(_pdl))
+        lib.dk_set_pdl.argtypes = lib.dk_set_thread_pdl.argtypes = [c_int]
+        lib.dk_set_pdl(int(bool(_pdl)))
         lib.dk_error_string.restype = ctypes.c_char_p
+    thread = _thread
+    want = thread.dependent if _pdl is None else _pdl
+    if thread.told.get(key) is not want:
+        lib.dk_set_thread_pdl(int(want))
+        thread.told[key] = want
     return lib
 
 
@@ -78,6 +115,8 @@ def launch_count():
 def _check(lib, err, what, kernels=1):
     global _launches
     _launches += kernels
+    if _thread.steps:
+        _thread.dependent = True
     if err != 0:
         msg = lib.dk_error_string(err).decode()
         raise KernelError(f"{what}: CUDA error {err} ({msg})")

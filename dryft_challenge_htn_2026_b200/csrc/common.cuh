@@ -83,8 +83,11 @@ __device__ __forceinline__ uint64_t l2_evict_first() {
     return p;
 }
 
-static int g_pdl = 0;
+static int g_pdl = 0;                     // for threads that have not chosen themselves
+static thread_local int t_pdl = -1;       // 1, 0: this thread's launches; -1: as g_pdl says
 DK_EXPORT void dk_set_pdl(int on) { g_pdl = on; }
+DK_EXPORT void dk_set_thread_pdl(int on) { t_pdl = on; }
+static inline bool pdl_on() { return (t_pdl >= 0 ? t_pdl : g_pdl) != 0; }
 
 template <typename... KArgs, typename... Args>
 static inline int dk_launch_as(bool dependent, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
@@ -110,7 +113,7 @@ static inline int dk_launch_as(bool dependent, void (*kernel)(KArgs...), dim3 gr
 
 template <typename... KArgs, typename... Args>
 static inline int dk_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
-    return dk_launch_as(g_pdl != 0, kernel, grid, block, smem, stream, args...);
+    return dk_launch_as(pdl_on(), kernel, grid, block, smem, stream, args...);
 }
 // For kernels of many rows, which run for tens of microseconds: a start under the end of the kernel before gains them nothing
 // (a prompt of 2,048 tokens: 16.36 ms with dependent launches throughout, 15.98 as without any).

@@ -673,7 +673,7 @@ int launch(const bf16* x, const bf16* W, bf16* out, int M, int N, int K, int* er
     e = make_map(&mw, W, MODE == 2 ? 2LL * N : N, K, MODE == 2 ? BN / 2 : BN);
     if (e) return e;
     // only the decode form (early_w in the kernel) has anything to do before the kernel in front of it ends
-    return dk_launch_as(g_pdl != 0 && (m_tiles == 1 || ws != nullptr), gemm_tc_kernel<BN, MODE>, dim3(units < sms ? units : sms), dim3(192), smem, st, mx, mw, out, M, N, K,
+    return dk_launch_as(pdl_on() && (m_tiles == 1 || ws != nullptr), gemm_tc_kernel<BN, MODE>, dim3(units < sms ? units : sms), dim3(192), smem, st, mx, mw, out, M, N, K,
                      m_tiles, tiles, group_m, err, SK, ws, stages, a_bytes, qe);
 }
 

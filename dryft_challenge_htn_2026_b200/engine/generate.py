@@ -206,9 +206,10 @@ class DecodeState:
         self.tok_copied.record()
 
     def body(self, advance=True, out_tok=None):
-        self.logits = self.runner.model.forward(self.ctx, self.runner.cache)
-        self.sampler(self.logits, self.temps, self.seeds, self.ctx.row_pos, None,
-                     self.ctx.tok if out_tok is None else out_tok, advance)
+        with api.dependent_launches():
+            self.logits = self.runner.model.forward(self.ctx, self.runner.cache)
+            self.sampler(self.logits, self.temps, self.seeds, self.ctx.row_pos, None,
+                         self.ctx.tok if out_tok is None else out_tok, advance)
 
     def capture(self):
         """Two plain runs that leave positions and tokens alone (they compile and size everything,

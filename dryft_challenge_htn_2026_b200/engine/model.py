@@ -137,6 +137,10 @@ class CausalLM:
         """``tap(k, h)``: called after the k-th schedule entry with the residual stream as it then
         stands (that entry's feed-forward output added in): for dumps that look for the layer where
         two runs part ways. It costs a launch and a copy per entry, so it is for debugging only."""
+        with api.dependent_launches():
+            return self._forward(ctx, cache, tap)
+
+    def _forward(self, ctx, cache, tap):
         s, rt = self.spec, self.rt
         h = torch.empty((ctx.n_tok, s.hidden_size), dtype=torch.float32, device=rt.device)
         a = torch.empty((ctx.n_tok, s.hidden_size), dtype=rt.dtype, device=rt.device)
