@@ -793,14 +793,16 @@ def gemm_tc_fills_gpu(M, N, min_fill=0.8):
 
 
 def gemm_tc_check():
-    """Raises if a bounded wait inside gemm_tc or attention_prefill_tc ran out since the last check (synchronises)."""
-    if _tc_err is not None:
+    """Raises if a bounded wait inside a tensor-core product or attention_prefill_tc ran out since the last check (synchronises; a
+    stream that is being captured cannot be asked)."""
+    if _tc_err is not None and not (_tc_err.is_cuda and torch.cuda.is_current_stream_capturing()):
         code = int(_tc_err.item())
         if code:
             _tc_err.zero_()
             for t in _attn_sched.values():
                 t.zero_()
-            raise KernelError(f"gemm_tc: a bounded wait ran out (code {code}); its results are not valid")
+            kernel = "gemm_f32_tc" if 11 <= code <= 15 else "gemm_tc or attention_prefill_tc"
+            raise KernelError(f"{kernel}: a bounded wait ran out (code {code}); its results are not valid")
 
 
 # --------------------------------------------------------------- tensor-core prefill attention

@@ -288,7 +288,8 @@ class DecodeLoop:
         """One token per sequence, given: entries [(slot, [token], want)]. Returns float32 logits of
         the entries whose ``want`` is not empty, in order. The state is filled anew when the
         sequences or their pages are not the ones it holds; otherwise only the tokens are written
-        and the positions are those the last step left on the device."""
+        and the positions are those the last step left on the device. Raises ``KernelError`` where a
+        kernel of the step gave up a wait."""
         cache = self.runner.cache
         for slot, tokens, _ in entries:
             if len(tokens) != 1:
@@ -305,6 +306,7 @@ class DecodeLoop:
         else:
             st.set_tokens([tokens[0] for _, tokens, _ in entries])
         self.run()
+        api.gemm_tc_check()
         rows = [i for i, (_, _, want) in enumerate(entries) if want]
         return st.logits[rows] if rows else st.logits[:0]
 

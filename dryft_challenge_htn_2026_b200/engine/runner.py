@@ -79,7 +79,8 @@ class Runner:
         """entries: list of (slot, tokens, want). Returns float32 logits [sum(len(want)), vocab]
         on the device, in the order of the entries and of each ``want``. ``tap``: see
         ``CausalLM.forward``. ``with_context``: also return the step's ``StepContext`` (the
-        generation loop samples from the logits with its positions and wanted rows).
+        generation loop samples from the logits with its positions and wanted rows). Raises ``KernelError``
+        where a kernel of the step gave up a wait, for which the step is waited for.
         ``graph``: a step shape that comes a second time is captured as a CUDA graph and replayed
         from then on (short steps are bound by the host's launches otherwise; the reference
         captures its prefill per length too: engine/engine.py:505-536). The logits of a replayed
@@ -92,8 +93,7 @@ class Runner:
         logits = self.model.forward(ctx, self.cache, tap)
         for slot, tokens, _ in entries:
             self.cache.commit(slot, len(tokens))
-        if not ctx.is_decode:
-            api.gemm_tc_check()
+        api.gemm_tc_check()      # single tokens too: their products wait within the kernel as well
         return (logits, ctx) if with_context else logits
 
     def _graph_step(self, entries, with_context):
@@ -125,6 +125,5 @@ class Runner:
         sg.graph.replay()
         for slot, tokens, _ in entries:
             self.cache.commit(slot, len(tokens))
-        if not sg.ctx.is_decode:
-            api.gemm_tc_check()
+        api.gemm_tc_check()
         return (sg.logits, sg.ctx) if with_context else sg.logits
