@@ -42,6 +42,15 @@ constexpr int EX_BYTES = 2 * 32 * 64 * 4, HALF_COLS = MAX_NT / 2;
 #ifndef DK_WAIT_CYCLES
 #define DK_WAIT_CYCLES 2000000000LL               // about a second: a wait this long has failed
 #endif
+#ifdef DK_TEST_STALL
+// Test build only: with the flag set no weights are requested, so the waits of all other roles run out (after DK_WAIT_CYCLES,
+// which such a build makes short): a code in *err, tensor memory given back, the kernel returns.
+__device__ int dk_stall_flag;
+DK_EXPORT int dk_test_stall(int on) { return (int)cudaMemcpyToSymbol(dk_stall_flag, &on, sizeof(int)); }
+#define DK_STALLED (dk_stall_flag != 0)
+#else
+#define DK_STALLED false
+#endif
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void mbar_init(uint64_t* bar, int count) {
@@ -244,7 +253,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
             const uint32_t tx = (MODE == 2 ? 2 : 1) * p.tile_n * 256;
             int s = 0, it = 0;
             uint32_t round = 0;
-            bool ok = true;
+            bool ok = !DK_STALLED;
             for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
                 UNIT(u);
                 for (int kb = kb0; kb < kb1; kb++, it++, s = s + 1 == p.w_stages ? 0 : s + 1, round ^= (s == 0)) {
@@ -387,7 +396,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
                 for (int kb = g0; kb < g1; kb++, it++) {
                     const int b = it & 1;
                     if (ok) ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[b], (it >> 1) & 1));
-                    if (!ok) {             // go on without waiting: the warps meet at barriers below
+                    if (!ok) {             // go on without waiting: the warps meet at barriers below, and the sums are not valid
                         atomicExch(err, 15);
                         continue;
                     }

@@ -16,12 +16,12 @@ TEST_BUILD = {"DK_TEST_STALL": 1, "DK_WAIT_CYCLES": "4000000LL"}      # about tw
 
 @pytest.fixture
 def stalled(monkeypatch):
-    """api._lib hands out the test builds of the two tensor-core sources; yields a switch for their flag."""
+    """api._lib hands out the test builds of the tensor-core sources; yields a switch for their flag."""
     real = api._lib
     libs = []
 
     def lib_for(source, defines=None):
-        if source in ("gemm_tc.cu", "attention_tc.cu"):
+        if source in ("gemm_tc.cu", "gemm_f32_tc.cu", "attention_tc.cu"):
             lib = real(source, dict(defines or {}, **TEST_BUILD))
             if lib not in libs:
                 libs.append(lib)
@@ -31,7 +31,7 @@ def stalled(monkeypatch):
     monkeypatch.setattr(api, "_lib", lib_for)
 
     def switch(on):
-        for source, defines in (("gemm_tc.cu", None), ("attention_tc.cu", {"HD": 128})):
+        for source, defines in (("gemm_tc.cu", None), ("gemm_f32_tc.cu", None), ("attention_tc.cu", {"HD": 128})):
             assert lib_for(source, defines).dk_test_stall(int(on)) == 0
     yield switch
     switch(False)
@@ -59,6 +59,36 @@ def test_a_product_whose_loads_never_come_reports_and_the_next_one_is_right(stal
     assert float((out.float() - ref).abs().max()) <= 0.02 * float(ref.abs().max())
     want = ref / (1 + torch.exp(-ref)) * ref
     assert float((g.float() - want).abs().max()) <= 0.03 * float(want.abs().max())
+
+
+def test_a_float32_product_whose_weights_never_come_reports_and_the_next_one_is_right(stalled):
+    """Whole tiles of more chunks than the rings hold, groups added into the output, groups left in parts, the gated form (whose
+    warps meet at barriers of their own), and a product so short that the loader of x never waits."""
+    x, w = torch.randn(150, 1088, device=DEV), torch.randn(300, 1088, device=DEV) * 0.05
+    ref = x.double() @ w.double().T
+    cases = [(x, w, api.MODE_STORE, None), (x, w, api.MODE_STORE, (32, 64, False)), (x, w, api.MODE_STORE, (128, 80, True)),
+             (x, w, api.MODE_SILU, None), (x[:2, :64].contiguous(), w[:, :64].contiguous(), api.MODE_STORE, None)]
+    assert api.f32_groups(300, 1088)[0] > 1
+
+    def run(x, w, mode, plan):
+        out = api.gemm_f32_tc(x, w, mode, plan)
+        return out.sum(torch.float32) if isinstance(out, api.Partial) else out
+
+    stalled(False)
+    good = [run(*c) for c in cases]
+    api.gemm_tc_check()
+    assert float((good[0].double() - ref).abs().max()) <= 1e-5 * float(ref.abs().max())
+    stalled(True)
+    for c in cases:
+        run(*c)
+        torch.cuda.synchronize()                                       # the kernel came back by itself
+        with pytest.raises(api.KernelError, match="gemm_f32_tc: a bounded wait.*1[1-5]"):
+            api.gemm_tc_check()
+        api.gemm_tc_check()
+    stalled(False)
+    for c, want in zip(cases, good):
+        assert torch.equal(run(*c), want)                              # tensor memory was given back, the barriers start anew
+    api.gemm_tc_check()
 
 
 def test_attention_whose_loads_never_come_reports_and_the_next_one_is_right(stalled):
