@@ -441,6 +441,7 @@ def f32_plan(M, N, K, mode=MODE_STORE, allow_partial=False):
     kb = (K + F32_CHUNK - 1) // F32_CHUNK
     groups, length = f32_groups(N, K, mode)
     per_out = 2 if mode == MODE_SILU else 1
+    M = max(M, 1)                     # no rows are planned as one
     fewest = (M + F32_MAX_ROW_TILE - 1) // F32_MAX_ROW_TILE
     best = None
     for row_tiles in range(fewest, fewest + 3):
@@ -474,6 +475,7 @@ def gemm_f32_tc(x, w, mode=MODE_STORE, plan=None, act=(0.0, 0.0), out=None):
     groups, length = f32_groups(N, K, mode)
     if split and (groups == 1 or mode in (MODE_SILU, MODE_XIELU) or out is not None):
         raise KernelError("gemm_f32_tc: nothing to split, or a result that cannot be left in parts")
+    split = split and M > 0
     ws = None
     if split:
         ws = torch.empty((groups, M, N), dtype=torch.float32, device=x.device)
@@ -481,6 +483,8 @@ def gemm_f32_tc(x, w, mode=MODE_STORE, plan=None, act=(0.0, 0.0), out=None):
         out = torch.empty((M, N), dtype=torch.float32, device=x.device)
     elif tuple(out.shape) != (M, N):
         raise KernelError(f"gemm_f32_tc: out {tuple(out.shape)} is not {(M, N)}")
+    if M == 0:
+        return out
     pieces = torch.empty(3 * M * ((K + 7) // 8 * 8), dtype=torch.bfloat16, device=x.device)
     if _tc_err is None:
         _tc_err = torch.zeros(1, dtype=torch.int32, device=x.device)
