@@ -3,7 +3,11 @@
 //   out[M,N] = silu(x . Wgate^T) * (x . Wup^T)          (mode 2, W = [gate; up], N rows each; the other gates as in gemm.cu)
 // A float32 number is the sum of three bfloat16 numbers (8 + 8 + 8 significant bits, each rounded to nearest, the
 // remainders exact), so x . w is the sum of nine exact bfloat16 products; the six largest are taken (the three left out
-// are below 2^-26 of |x w|). What limits the result is then the accumulator of the tensor cores, so it never holds more
+// are below 2^-26 of |x w|). The second and third piece are kept 2^8 and 2^16 times as large, so that they do not fall under
+// bfloat16's range before the number itself does (without, the error of numbers below 2^-110 grew to 2e-3 at 2^-126; now only
+// subnormal numbers below 2^-133, whose first piece is 0, meet the other operand's first 8 to 16 bits alone); the
+// accumulator then holds 2^16 times the sums of the smallest products, 2^8 times the next ones', and the mma that goes on
+// to larger ones scales it down (scale-input-d). What limits the result is then the accumulator of the tensor cores, so it never holds more
 // than 64 columns of K: within such a chunk the small products go first and the large ones last (four additions at full
 // size), and the chunk's sums are drained from tensor memory and added up in float32 registers, in order. The error
 // against float64 (2-norm, relative) is 0.8e-7 at K = 64, 1.1e-7 at 2,560 and 1.3e-7 at 9,728, where one float32 FMA chain over K
@@ -23,9 +27,9 @@
 //   warps 8-15  drain: two threads a row, half of the columns each, add up the two accumulators in turn; epilogue.
 //   warp 16     TMA of the weights; warp 17 tcgen05.mma; warp 18 TMA of the pieces of x ([3][M][Kp] bfloat16, made by
 //               split_rows before: as the B operand they come ready from shared memory).
-// Measured in a graph (2,560 wide layers of 9,728; sgemm -> this kernel with split_rows): 544 rows: q/k/v 740 -> 117 us, output
-// projection 609 -> 100, gated 1,994 -> 344, down 1,455 -> 166 (160 TFLOP/s; without the mma the gated product takes 231: the
-// tiles' 75 KB a chunk from the L2 and the mma overlap in part only). One row: 175 -> 16, 273 -> 14, 409 -> 59, 839 -> 23, a
+// Measured in a graph (2,560 wide layers of 9,728; sgemm -> this kernel with split_rows): 544 rows: q/k/v 740 -> 113 us, output
+// projection 609 -> 97, gated 1,994 -> 349, down 1,455 -> 163 (165 TFLOP/s; without the mma the gated product takes 231: the
+// tiles' 75 KB a chunk from the L2 and the mma overlap in part only). One row: 175 -> 14, 273 -> 11, 409 -> 57, 839 -> 19, a
 // head of 151,936 1,733 -> 260 (6.0 TB/s).
 // Infinities, NaN and numbers beyond bfloat16's largest: a piece times a zero piece is NaN where the product is not. A
 // thread that finds a sum that is not finite works that one out again by plain FMA from x and W.
@@ -102,6 +106,13 @@ __device__ __forceinline__ void umma_ts(uint32_t d, uint32_t a_tmem, uint64_t b,
                  "r"(a_tmem), "l"(b), "r"(idesc), "r"(acc)
                  : "memory");
 }
+// The same onto the accumulator times 2^-8.
+__device__ __forceinline__ void umma_ts_down8(uint32_t d, uint32_t a_tmem, uint64_t b, uint32_t idesc) {
+    asm volatile(
+        "{ .reg .pred p; setp.ne.b32 p, 1, 0; tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%4, %4, %4, %4}, p, 8; }" ::"r"(d),
+        "r"(a_tmem), "l"(b), "r"(idesc), "r"(0)
+        : "memory");
+}
 // One lane of a converged warp. The compiler keeps the operands of an mma issued under it in uniform registers; under
 // ``lane == 0`` it moves every one of them there first, 80 clocks an mma instead of 50 (the head's product of one row: 601 us
 // instead of 343).
@@ -129,15 +140,30 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16
         : "memory");
 }
 
-// The three bfloat16 pieces of a and b, packed in pairs (a in the low half).
+// What a pair (two float32 in one register pair) has left beside its rounding to bfloat16, times 2^8; exact.
+__device__ __forceinline__ void remainder_up8(uint64_t& pair, uint32_t rounded) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(rounded << 16), "r"(rounded & 0xffff0000u));
+    asm("sub.rn.f32x2 %0, %0, %1;" : "+l"(pair) : "l"(r));
+    asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(pair) : "l"(0x4380000043800000ull));
+}
+__device__ __forceinline__ uint32_t round_pair(uint64_t pair) {
+    uint32_t lo, hi, out;
+    asm("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "l"(pair));
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(out) : "f"(__uint_as_float(hi)), "f"(__uint_as_float(lo)));
+    return out;
+}
+// The three bfloat16 pieces of a and b, packed in pairs (a in the low half): a = hi + mid / 2^8 + lo / 2^16. Two numbers an
+// instruction: with one at a time two sequences generating 12 tokens took 71.5 ms instead of 66.2 unscaled; a gated product of one
+// row takes 57.2 us (56.0 unscaled).
 __device__ __forceinline__ void split_pair(float a, float b, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
-    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(hi) : "f"(b), "f"(a));
-    a -= __uint_as_float(hi << 16);
-    b -= __uint_as_float(hi & 0xffff0000u);
-    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(mid) : "f"(b), "f"(a));
-    a -= __uint_as_float(mid << 16);
-    b -= __uint_as_float(mid & 0xffff0000u);
-    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(lo) : "f"(b), "f"(a));
+    uint64_t pair;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(pair) : "r"(__float_as_uint(a)), "r"(__float_as_uint(b)));
+    hi = round_pair(pair);
+    remainder_up8(pair, hi);
+    mid = round_pair(pair);
+    remainder_up8(pair, mid);
+    lo = round_pair(pair);
 }
 
 // x [M][K] float32 -> pieces [3][M][Kp] bfloat16, Kp = K rounded up to 8, zeros behind K. A thread takes 8 columns.
@@ -321,13 +347,17 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
                 if (elect_one()) {
                     const uint32_t d = tmem + b * MAX_NT, a = tmem + A_BASE + b * A_COLS;
                     const uint32_t xb = smem_u32(smem_x + xs * x_stage);
-                    // (piece of W, piece of x), 0 the largest; the products grow from the first to the last
+                    // (piece of W, piece of x), 0 the largest; the products grow from the first to the last, at 2^16, 2^8 and 1
                     constexpr int PA[6] = {2, 0, 1, 1, 0, 0}, PB[6] = {0, 2, 1, 0, 1, 0};
 #pragma unroll
                     for (int q = 0; q < 6; q++)
 #pragma unroll
-                        for (int k = 0; k < BK / 16; k++)
-                            umma_ts(d, a + PA[q] * 32 + k * 8, umma_desc(xb + PB[q] * x_piece + k * 32), idesc, (q | k) != 0);
+                        for (int k = 0; k < BK / 16; k++) {
+                            const uint32_t ak = a + PA[q] * 32 + k * 8;
+                            const uint64_t bk = umma_desc(xb + PB[q] * x_piece + k * 32);
+                            if (k == 0 && q > 0 && PA[q] + PB[q] < PA[q - 1] + PB[q - 1]) umma_ts_down8(d, ak, bk, idesc);
+                            else umma_ts(d, ak, bk, idesc, (q | k) != 0);
+                        }
                     umma_commit(&x_empty[xs]);
                     umma_commit(&a_empty[b]);
                     umma_commit(&acc_full[b]);

@@ -77,3 +77,17 @@ def test_refusals():
         api.gemm_f32_tc(x, rnd(8 * 64 + 1, seed=9)[1:].view(8, 64))
     with pytest.raises(api.KernelError):
         api.gemm_f32_tc(x, w, plan=(32, 16, True))
+
+
+@pytest.mark.parametrize("ex,ew", [(-115, 0), (-120, 0), (-126, 0), (-130, 5), (-140, 20), (0, -125), (100, -120), (115, 2), (-60, -60)])
+def test_small_and_large_numbers_keep_their_bits(ex, ew):
+    """Numbers near and under 2^-126, whose second and third piece bfloat16 has no room for as they stand, and large ones: the error
+    (2-norm, relative) that K = 1,024 has at any size, below sgemm's. Numbers under 2^-133 have no first piece: their largest is the
+    second or the third, and of the products the one with the other operand's third, or second and third, is not taken: 2^-9 of
+    such a term at most (the other operand rounded to its first 8 bits)."""
+    x, w = rnd(8, 1024, seed=10, scale=2.0 ** ex), rnd(256, 1024, seed=11, scale=2.0 ** ew)
+    ref = x.double() @ w.double().T
+    out = torch.empty(8, 256, device=DEV)
+    api.sgemm(x, w, out)
+    err = [float((o.double() - ref).norm() / ref.norm()) for o in (api.gemm_f32_tc(x, w), out)]
+    assert err[0] <= (2.0 ** -9 if ex < -133 else min(err[1], 3e-7)), err
