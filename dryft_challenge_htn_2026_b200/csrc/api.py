@@ -415,6 +415,7 @@ def sgemm(x, w, out, mode=MODE_STORE, act=(0.0, 0.0)):
 F32_TC_MIN_K = 256
 F32_CHUNK = 64              # columns of K that gemm_f32_tc adds up in tensor memory at a time
 F32_MAX_ROW_TILE = 128      # rows of x a tile
+F32_PIECES_BYTES = 256 << 20  # most scratch memory for the pieces of x; more rows go in several launches
 F32_TILE_HEIGHTS = (128, 112, 96, 80, 64, 56, 48, 40, 32)      # outputs a tile (the gated product: half of them)
 
 
@@ -452,13 +453,21 @@ def f32_plan(M, N, K, mode=MODE_STORE, allow_partial=False):
             bytes_w = per_out * tile_n * 256
             chunk = max(24 * max(nt / 2, 50), bytes_w / 24 / row_tiles, (bytes_w + 384 * nt) / 40)
             tiles = (N + tile_n - 1) // tile_n
-            for split in ((False, True) if allow_partial and groups > 1 else (False,)):
+            for split in ((False, True) if allow_partial and groups > 1 and f32_rows_a_launch(M, K) == M else (False,)):
                 units = tiles * row_tiles * (groups if split else 1)
                 unit = (length if split else kb) * chunk + 2500 + (0 if split else (groups - 1) * 1500)
                 cost = -(-units // sms) * unit + (groups * M * N * 8 / (sms * 24) if split else 0)
                 if best is None or cost < best[0]:
                     best = cost, (tile_n, nt, split)
     return best[1]
+
+
+def f32_rows_a_launch(M, K):
+    """Rows of x that gemm_f32_tc takes apart at a time: all, or equal shares of whole row tiles whose pieces, 6 bytes a number,
+    fit F32_PIECES_BYTES (4,480 rows at K = 9,728; a row's result does not depend on the rows beside it)."""
+    most = max(1, F32_PIECES_BYTES // (6 * ((K + 7) // 8 * 8 * F32_MAX_ROW_TILE))) * F32_MAX_ROW_TILE
+    launches = -(-M // most)
+    return M if launches <= 1 else -(-M // (launches * F32_MAX_ROW_TILE)) * F32_MAX_ROW_TILE
 
 
 def gemm_f32_tc(x, w, mode=MODE_STORE, plan=None, act=(0.0, 0.0), out=None):
@@ -485,12 +494,16 @@ def gemm_f32_tc(x, w, mode=MODE_STORE, plan=None, act=(0.0, 0.0), out=None):
         raise KernelError(f"gemm_f32_tc: out {tuple(out.shape)} is not {(M, N)}")
     if M == 0:
         return out
-    pieces = torch.empty(3 * M * ((K + 7) // 8 * 8), dtype=torch.bfloat16, device=x.device)
+    rows = M if split else f32_rows_a_launch(M, K)
+    pieces = torch.empty(3 * rows * ((K + 7) // 8 * 8), dtype=torch.bfloat16, device=x.device)
     if _tc_err is None:
         _tc_err = torch.zeros(1, dtype=torch.int32, device=x.device)
     lib = _lib("gemm_f32_tc.cu")
-    _check(lib, lib.dk_gemm_f32_tc(_p(x), _p(w), _p(out), _p(pieces), M, N, K, 0 if mode == MODE_STORE_F32 else mode, groups, length,
-                                   _p(ws), tile_n, nt, _p(_tc_err), c_float(act[0]), c_float(act[1]), _stream()), "gemm_f32_tc", 2)
+    for m in range(0, M, rows):
+        _check(lib, lib.dk_gemm_f32_tc(c_void_p(x.data_ptr() + 4 * m * K), _p(w), c_void_p(0 if split else out.data_ptr() + 4 * m * N),
+                                       _p(pieces), min(rows, M - m), N, K, 0 if mode == MODE_STORE_F32 else mode,
+                                       groups, length, _p(ws), tile_n, nt, _p(_tc_err), c_float(act[0]), c_float(act[1]),
+                                       _stream()), "gemm_f32_tc", 2)
     return Partial(ws) if split else out
 
 

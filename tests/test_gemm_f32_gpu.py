@@ -91,3 +91,16 @@ def test_small_and_large_numbers_keep_their_bits(ex, ew):
     api.sgemm(x, w, out)
     err = [float((o.double() - ref).norm() / ref.norm()) for o in (api.gemm_f32_tc(x, w), out)]
     assert err[0] <= (2.0 ** -9 if ex < -133 else min(err[1], 3e-7)), err
+
+
+@pytest.mark.parametrize("mode", [api.MODE_STORE, api.MODE_SILU, api.MODE_XIELU])
+@pytest.mark.parametrize("M", [256, 257, 700])
+def test_rows_in_several_launches(monkeypatch, mode, M):
+    """The bits of one launch, whatever the share of rows a launch takes (here one tile of 128)."""
+    x, w = rnd(M, 1028, seed=12), rnd(2 * 72, 1028, seed=13, scale=0.1)
+    whole = api.gemm_f32_tc(x, w, mode, act=(0.7, 0.3) if mode == api.MODE_XIELU else (0.0, 0.0))
+    monkeypatch.setattr(api, "F32_PIECES_BYTES", 6 * 1032 * 128)
+    assert api.f32_rows_a_launch(M, 1028) == 128 and api.f32_rows_a_launch(128, 1028) == 128
+    cut = api.gemm_f32_tc(x, w, mode, (64, 64, False), act=(0.7, 0.3) if mode == api.MODE_XIELU else (0.0, 0.0))
+    assert torch.equal(cut, whole)
+    api.gemm_tc_check()

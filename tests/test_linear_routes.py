@@ -14,3 +14,54 @@ def test_no_rows_in_float32_give_no_rows(monkeypatch, K, mode, allow_partial):
     monkeypatch.setattr(api, "_need", lambda *a: None)
     out = linear(torch.empty(0, K), torch.empty(40, K), mode, allow_partial=allow_partial and mode in (STORE, STORE_F32))
     assert isinstance(out, torch.Tensor) and out.dtype == torch.float32 and tuple(out.shape) == (0, 20 if mode == SILU else 40)
+
+
+class _Launches:
+    """A library that notes the arguments of its launches."""
+
+    def __init__(self):
+        self.calls = []
+
+    def __getattr__(self, name):
+        def call(*args):
+            self.calls.append((name, [a.value if hasattr(a, "value") else a for a in args]))
+            return 0
+        return call
+
+
+@pytest.fixture
+def launches(monkeypatch):
+    lib, sizes, empty = _Launches(), [], torch.empty
+
+    def noted(*shape, **kw):
+        out = empty(*shape, **kw)
+        sizes.append(out.numel() * out.element_size())
+        return out
+
+    monkeypatch.setattr(api, "_need", lambda *a: None)
+    monkeypatch.setattr(api, "_lib", lambda source, defines=None: lib)
+    monkeypatch.setattr(api, "_stream", lambda: None)
+    monkeypatch.setattr(api, "_tc_err", torch.zeros(1, dtype=torch.int32))
+    monkeypatch.setattr(torch, "empty", noted)
+    lib.sizes = sizes
+    return lib
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 64, 256), (544, 96, 9728), (9000, 32, 9728), (30000, 8, 4100), (4609, 24, 9732)])
+@pytest.mark.parametrize("partial", [False, True])
+def test_scratch_of_the_float32_product_is_bounded(launches, M, N, K, partial):
+    """However many rows: at most 256 MB of pieces, every row in one launch, in order, the pieces' buffer the same for all."""
+    x = torch.zeros(1).expand(M, K)          # no memory of its own: nothing is read here
+    out = linear(x, torch.zeros(1).expand(N, K), STORE, allow_partial=partial)
+    assert max(launches.sizes) <= max(256 << 20, 4 * M * N * (api.f32_groups(N, K)[0] if isinstance(out, api.Partial) else 1))
+    at = 0
+    for name, a in launches.calls:
+        rows = a[4]
+        assert name == "dk_gemm_f32_tc" and a[0] == x.data_ptr() + 4 * at * K and a[3] == launches.calls[0][1][3]
+        assert 6 * rows * ((K + 7) // 8 * 8) <= 256 << 20 and 3 * rows <= 1 << 30
+        if not isinstance(out, api.Partial):
+            assert a[2] == out.data_ptr() + 4 * at * N and tuple(out.shape) == (M, N)
+        else:
+            assert len(launches.calls) == 1 and rows == M
+        at += rows
+    assert at == M
