@@ -522,7 +522,10 @@ DK_EXPORT int dk_add_rmsnorm(int dtype, float* h, const void* delta, const float
     if (dtype == 1 && parts == nullptr && rows == nullptr && H % 8 == 0 && H <= 8 * 4 * row_threads(H) && n_rows > 64)
         return dk_launch_whole(add_rmsnorm_wide_kernel, dim3(n_rows), dim3(row_threads(H)), 0, st, h, (const bf16*)delta, w, eps,
                          H, (bf16*)a);
-    if ((n_rows <= 64 || parts != nullptr) && H % 4 == 0 && H <= 8192 && part_stride % 4 == 0) {
+    // float32: this kernel at any number of rows and with or without parts, so that a row's sum of squares is added up in one
+    // order however many rows are beside it (its products are planned to leave parts at some row counts and not at others)
+    const bool dense32 = dtype == 0 && (((uintptr_t)h | (uintptr_t)delta | (uintptr_t)parts | (uintptr_t)w | (uintptr_t)a) & 15) == 0;
+    if ((n_rows <= 64 || parts != nullptr || dense32) && H % 4 == 0 && H <= 8192 && part_stride % 4 == 0) {
         if (H <= 4096) {
             DISPATCH_T(dtype, return dk_launch(add_rmsnorm_quad_kernel<T, 1>, dim3(n_rows), dim3((H / 4 + 31) / 32 * 32), 0, st, h,
                                                (const T*)delta, parts, n_parts, (size_t)part_stride, rows, w, eps, H, (T*)a));
