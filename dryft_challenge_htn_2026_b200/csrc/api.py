@@ -277,6 +277,7 @@ def attention_generic(q, out, k_store, v_store, row_pos, row_seq, page_table, n_
 
 F32_ATTENTION_HEAD_DIMS = (64, 128)
 F32_ATTENTION_MAX_GROUP = 16        # query heads a kv head
+F32_DECODE_BYTES = 256 << 20        # most scratch memory for the pages' results of single tokens; more sequences go in several launches
 F32_TILE_ROWS = 64                  # rows (queries x the query heads of a kv head) a block of attention_prompt_f32 takes
 
 
@@ -300,16 +301,21 @@ def attention_prompt_f32(q, out, k_store, v_store, tiles, cu_q, seq_pos0, page_t
 
 
 def attention_decode_f32(q, out, k_store, v_store, row_pos, page_table, n_heads, n_kv_heads, head_dim, window, scale):
-    """Float32 attention of one token a sequence (head sizes 64 and 128): a block a page of keys, merged in order by a second kernel."""
+    """Float32 attention of one token a sequence (head sizes 64 and 128): a block a page of keys, merged in order by a second kernel.
+    Up to F32_DECODE_BYTES of results a page are kept at a time."""
     _need_f32_attention(q, out, k_store, v_store, page_table, n_heads, n_kv_heads, head_dim)
     _need(row_pos, "row_pos", torch.int32, 1)
     n_seq, pages = q.shape[0], page_table.shape[1]
-    ws = torch.empty(n_seq * n_heads * pages * (head_dim + 2), dtype=torch.float32, device=q.device)
-    cut = n_seq * n_heads * pages * head_dim
+    share = max(1, min(n_seq, F32_DECODE_BYTES // (4 * n_heads * pages * (head_dim + 2)), 65535))
+    ws = torch.empty(share * n_heads * pages * (head_dim + 2), dtype=torch.float32, device=q.device)
+    cut = share * n_heads * pages * head_dim
     lib = _lib("attention_f32.cu", {"HD": head_dim})
-    _check(lib, lib.dk_attn_f32_decode(_p(q), _p(out), _p(k_store), _p(v_store), _p(row_pos), _p(page_table), pages, n_seq, n_heads,
-                                       n_kv_heads, int(window or 0), c_float(scale), _p(ws), _p(ws[cut:]), _stream()),
-           "attention_decode_f32", 2)
+    for i in range(0, n_seq, share):
+        at = 4 * i * n_heads * head_dim
+        _check(lib, lib.dk_attn_f32_decode(c_void_p(q.data_ptr() + at), c_void_p(out.data_ptr() + at), _p(k_store), _p(v_store),
+                                           c_void_p(row_pos.data_ptr() + 4 * i), c_void_p(page_table.data_ptr() + 4 * i * pages),
+                                           pages, min(share, n_seq - i), n_heads, n_kv_heads, int(window or 0), c_float(scale),
+                                           _p(ws), _p(ws[cut:]), _stream()), "attention_decode_f32", 2)
 
 
 def _attn_lib(head_dim):

@@ -51,6 +51,19 @@ def test_attention_f32(nh, nkv, hd, window):
     assert torch.equal(one[keep], out[rows][keep])
 
 
+@pytest.mark.parametrize("share", [1, 2, 4])
+def test_sequences_in_several_launches(monkeypatch, share):
+    """The bits of one launch, whatever the share of sequences a launch takes."""
+    nh, nkv, hd, before = 4, 2, 64, [0, 100, 63, 640, 64, 5, 200]
+    s = paged_setup(before, [1] * 7, nkv, hd, torch.float32, seed=13)
+    q, out = rnd(7, nh * hd, seed=14), []
+    for limit in (api.F32_DECODE_BYTES, share * 4 * nh * s["table"].shape[1] * (hd + 2)):
+        monkeypatch.setattr(api, "F32_DECODE_BYTES", limit)
+        out.append(torch.empty_like(q))
+        api.attention_decode_f32(q, out[-1], s["k_store"], s["v_store"], s["row_pos"], s["table"], nh, nkv, hd, 0, hd ** -0.5)
+    assert torch.equal(out[0], out[1])
+
+
 def test_refusals():
     s = paged_setup([0], [3], 1, 32, torch.float32, seed=7)
     q = rnd(3, 64, seed=8)

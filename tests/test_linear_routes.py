@@ -65,3 +65,22 @@ def test_scratch_of_the_float32_product_is_bounded(launches, M, N, K, partial):
             assert len(launches.calls) == 1 and rows == M
         at += rows
     assert at == M
+
+
+@pytest.mark.parametrize("n,nh,nkv,hd,pages", [(1, 32, 8, 128, 4), (0, 32, 8, 128, 4), (64, 32, 8, 128, 1024), (16, 128, 8, 64, 16384),
+                                               (70000, 2, 2, 64, 1)])
+def test_scratch_of_the_float32_decode_attention_is_bounded(launches, n, nh, nkv, hd, pages):
+    """However many sequences and pages: 256 MB of pages' results, or one sequence's; every sequence in one launch, in order."""
+    q, store, pos = torch.zeros(1).expand(n, nh * hd), torch.zeros(1), torch.zeros(1, dtype=torch.int32)
+    table = pos.expand(n, pages)
+    api.attention_decode_f32(q, q, store, store, pos, table, nh, nkv, hd, 0, 0.1)
+    one = 4 * nh * pages * (hd + 2)
+    assert max(launches.sizes) <= max(256 << 20, one)
+    at = 0
+    for name, a in launches.calls:
+        assert name == "dk_attn_f32_decode" and a[0] == a[1] == q.data_ptr() + 4 * at * nh * hd
+        assert a[4] == pos.data_ptr() + 4 * at and a[5] == table.data_ptr() + 4 * at * pages
+        assert a[7] <= 65535 and one * a[7] <= max(256 << 20, one)
+        assert a[13] - a[12] == 4 * min(n, launches.sizes[0] // one) * nh * pages * hd
+        at += a[7]
+    assert at == n
