@@ -80,8 +80,8 @@ __device__ __forceinline__ void weights(float (&s)[4], float scale, int key0, in
     for (int o = 8; o > 0; o >>= 1) mp = fmaxf(mp, __shfl_xor_sync(0xffffffffu, mp, o));
 #pragma unroll
     for (int j = 0; j < 4; j++) {
-        const int key = key0 + tx + 16 * j;
-        s[j] = key >= lo && key <= pos ? expf(__fsub_rn(s[j], mp)) : 0.f;
+        // -inf: a key out of sight, or one whose score is; in a page of none but those, -inf - mp would be NaN
+        s[j] = s[j] == -INFINITY ? 0.f : expf(__fsub_rn(s[j], mp));
     }
     lp = __fadd_rn(__fadd_rn(__fadd_rn(s[0], s[1]), s[2]), s[3]);
 #pragma unroll

@@ -51,6 +51,40 @@ def test_attention_f32(nh, nkv, hd, window):
     assert torch.equal(one[keep], out[rows][keep])
 
 
+@pytest.mark.parametrize("hd", [64, 128])
+def test_pages_of_keys_with_infinitely_low_scores(hd):
+    """Keys whose score is -inf weigh nothing, also where a page holds (or shows a query) no others: before, between and after
+    pages with finite ones, as a page's first visible key, and NaN and +inf still come through."""
+    n = 200
+    s = paged_setup([0], [n], 1, hd, torch.float32, seed=11)
+    q = rnd(n, 2 * hd, seed=12).abs() + 0.1             # positive: a key of -inf scores -inf
+    low = [slice(0, 64), slice(100, 128), slice(128, 192)]
+    page = s["table"][0].long()
+    for part in low:
+        for j in range(part.start, part.stop):
+            s["k_store"][page[j // 64], 0, j % 64] = float("-inf")
+            s["dense_k"][0][j, 0] = float("-inf")
+    plan = QueryTiles(api.F32_TILE_ROWS // 2).build([n], [0], False)
+
+    def both():
+        out, one = torch.empty_like(q), torch.empty_like(q)
+        api.attention_prompt_f32(q, out, s["k_store"], s["v_store"], torch.tensor(plan, device=DEV), s["cu_q"], s["pos0"], s["table"],
+                                 2, 1, hd, 0, hd ** -0.5)
+        api.attention_decode_f32(q, one, s["k_store"], s["v_store"], s["row_pos"], s["table"].expand(n, -1).contiguous(), 2, 1, hd, 0,
+                                 hd ** -0.5)
+        return out, one
+
+    out, one = both()
+    ref = ref64(q, s, 2, 1, hd, 0)
+    assert bool(out[:64].isnan().all()) and bool(ref[:64].isnan().all())           # none but -inf in sight: 0 / 0
+    assert float((out[64:].double() - ref[64:]).abs().max()) <= 2e-5 * 4.5         # the bound of the test above
+    assert torch.equal(one[64:], out[64:]) and bool(one[:64].isnan().all())
+    for value in (float("nan"), float("inf")):
+        s["k_store"][page[2], 0, 5] = value                                       # position 133, in a page of -inf
+        out, one = both()
+        assert bool(out[133:].isnan().all()) and bool(one[133:].isnan().all()) and not bool(out[64:133].isnan().any())
+
+
 @pytest.mark.parametrize("share", [1, 2, 4])
 def test_sequences_in_several_launches(monkeypatch, share):
     """The bits of one launch, whatever the share of sequences a launch takes."""
