@@ -553,6 +553,7 @@ def _stream_smem(rows, K, sk, warps):
     return warps * 2 * 16 * (256 * 2 + 16) + 2 * warps * 16 * mr * 4 + mr * (per * 2 + 16)
 
 
+@functools.lru_cache(maxsize=4096)
 def stream_plan(M, N, K, mode, allow_partial=False):
     """(slices of K, blocks, streaming warps a block) for gemv_stream, or None if it cannot take
     the shape. Four warps and two persistent blocks per SM while the rows of x leave room for two
@@ -596,8 +597,9 @@ def stream_plan(M, N, K, mode, allow_partial=False):
 STREAM_SMALL_WEIGHTS = 8 << 20              # numbers of a matrix below which few rows always take the streaming product
 
 
-def few_rows_stream_plan(M, N, K, mode, allow_partial=False):
-    """The streaming product's plan for up to STREAM_BEST_ROWS rows, or None where the tensor-core product in its decode form
+@functools.lru_cache(maxsize=4096)
+def few_rows_plan(M, N, K, mode, allow_partial=False):
+    """(the streaming product's plan for up to STREAM_BEST_ROWS rows, whether its sums leave as a single float32 part), or (None, False) where the tensor-core product in its decode form
     (``skinny_tc_plan``) is the faster one: products that may stay in parts and are at least as deep as wide (a layer's output
     and down projections). While whole rows of x fit they stream in one slice with eight warps a block, since every slice costs the
     norm behind it (2,560 outputs of 4,096 at 8 rows, in a chain norm - product: 8.7 us, 9.4 in four slices as two blocks an SM,
@@ -605,14 +607,19 @@ def few_rows_stream_plan(M, N, K, mode, allow_partial=False):
     4,096 of 12,288: 24.0 -> 22.2; 5,120 of 17,408: 39.0 -> 35.1). Generation with both: one sequence of 4B sizes 69.2 -> 67.0 ms,
     eight 252 -> 242, three of 8B sizes 98.2 -> 96.0. The gated and the q/k/v product are as fast or faster there alone (21.2 against 22.3
     us, 8.9 against 9.1), but whole generations were 1 to 4 % slower with them on the tensor cores: their blocks take an SM's whole
-    shared memory, which the attention and rotation between them then wait for. Small matrices stay with ``stream_plan``. Sums that
-    left in parts, in float32, still do: one slice is one part (``linear``)."""
+    shared memory, which the attention and rotation between them then wait for. Small matrices stay with ``stream_plan``. Where it would
+    have cut a product into slices, whose sums go on in float32, the one slice that takes their place goes on in float32 too."""
     if allow_partial and mode in (MODE_STORE, MODE_STORE_F32) and N <= K and N * K >= STREAM_SMALL_WEIGHTS:
         if _stream_smem(M, K, 1, 8) <= _STREAM_SMEM_BLOCK:
-            return 1, sm_count(), 8
+            return (1, sm_count(), 8), True
         if skinny_tc_plan(M, N, K, MODE_STORE, True)[1] > 1:
-            return None
-    return stream_plan(M, N, K, mode, allow_partial)
+            return None, False
+    return stream_plan(M, N, K, mode, allow_partial), False
+
+
+def few_rows_stream_plan(M, N, K, mode, allow_partial=False):
+    """The plan alone."""
+    return few_rows_plan(M, N, K, mode, allow_partial)[0]
 
 
 def gemv_stream(x, w, out=None, mode=MODE_STORE, plan=None, act=(0.0, 0.0)):
@@ -731,6 +738,7 @@ TC_SKINNY_MAX_ROWS = 128
 TC_TILE_HEIGHTS = (128, 144, 160, 176, 192, 208, 224, 240, 256)   # weight rows a tile of gemm_tc
 
 
+@functools.lru_cache(maxsize=4096)
 def skinny_tc_plan(M, N, K, mode, allow_partial=False):
     """(weight rows per tile, slices of K) for gemm_tc on a decode step of up to 128 rows. A unit of
     work is (tile, slice), with a block of its own while the units fit the SMs; all blocks stream

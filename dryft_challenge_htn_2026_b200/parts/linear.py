@@ -3,7 +3,7 @@
 float32: the tensor-core product of three bfloat16 pieces (24 significant bits; gemm_f32_tc.cu) from an inner size of
 256 on, the CUDA-core sgemm below and where rows do not sit on 16-byte boundaries; which of the two depends on the weight
 alone, so a row's result never depends on the rows beside it. bfloat16: up to 8 rows the
-streaming kernel (cp.async rings, weights read once) where it is the faster one (``csrc.api.few_rows_stream_plan``); up to
+streaming kernel (cp.async rings, weights read once) where it is the faster one (``csrc.api.few_rows_plan``); up to
 128 rows the TMA + tcgen05 kernel in its decode form (one tile of rows, K in slices); for more rows (prefill) the same kernel, always for the
 gated product (SiLU*up fused into its epilogue) and otherwise when its 128 x 256 tiles fill the
 GPU's waves, else the library matrix product (the reference uses the library for all of these,
@@ -51,9 +51,8 @@ def linear(x, w, mode=STORE, allow_partial=False, act=(0.0, 0.0)):
             api.xielu(out, out, act[0], act[1])
         return out
     if M <= api.STREAM_BEST_ROWS and K % 16 == 0:
-        plan = api.few_rows_stream_plan(M, N, K, mode, allow_partial)
-        if plan is not None and plan[0] == 1 and mode == STORE and plan != api.stream_plan(M, N, K, mode, allow_partial):
-            # one slice where there were several: its float32 sums go on as the only part, not rounded in between
+        plan, one_part = api.few_rows_plan(M, N, K, mode, allow_partial)
+        if one_part and mode == STORE:
             return api.Partial(api.gemv_stream(x, w, None, STORE_F32, plan, act).unsqueeze(0))
         if plan is not None:
             return api.gemv_stream(x, w, None, mode, plan, act)

@@ -84,3 +84,44 @@ def test_scratch_of_the_float32_decode_attention_is_bounded(launches, n, nh, nkv
         assert a[13] - a[12] == 4 * min(n, launches.sizes[0] // one) * nh * pages * hd
         at += a[7]
     assert at == n
+
+
+LAYER = [(6144, 2560, STORE, True), (2560, 4096, STORE, True), (9728, 2560, SILU, False), (2560, 9728, STORE, True),
+         (151936, 2560, STORE_F32, False)]
+
+
+@pytest.mark.parametrize("M", [1, 8, 16])
+def test_a_product_of_a_shape_seen_before_is_not_planned_again(launches, monkeypatch, M):
+    """Every plainly launched step of few rows pays for its plans on the host, layer by layer."""
+    made = [0]
+    real = {name: getattr(api, name) for name in ("_stream_smem", "_few_units_plan")}
+
+    def counted(name):
+        def fn(*a):
+            made[0] += 1
+            return real[name](*a)
+        return fn
+
+    for name in real:
+        monkeypatch.setattr(api, name, counted(name))
+    w = torch.zeros(1, dtype=torch.bfloat16)
+    products = [(torch.zeros(M, K, dtype=torch.bfloat16), w.expand(2 * N if mode == SILU else N, K), mode, partial)
+                for N, K, mode, partial in LAYER]
+    for x, weights, mode, partial in products:
+        linear(x, weights, mode, partial)
+    made[0] = 0
+    for x, weights, mode, partial in products:
+        linear(x, weights, mode, partial)
+    streamed = sum(name == "dk_gemv_stream" for name, _ in launches.calls) // 2
+    assert made[0] == streamed                          # gemv_stream's look at the plan it is given, and nothing else
+
+
+def test_one_slice_goes_on_in_float32_exactly_where_it_takes_the_place_of_several():
+    for M in (1, 8):
+        for N in (72, 2560, 4096, 5120):
+            for K in (304, 2560, 2896, 4096, 5120, 5568, 9728):
+                for mode in (STORE, STORE_F32):
+                    for partial in (False, True):
+                        plan, one = api.few_rows_plan(M, N, K, mode, partial)
+                        several = plan is not None and plan[0] == 1 and (api.stream_plan(M, N, K, mode, partial) or (1,))[0] > 1
+                        assert one == several, (M, N, K, mode, partial)
