@@ -23,3 +23,12 @@ def pytest_collection_modifyitems(config, items):
     for item in items:
         if "gpu" in item.keywords:
             item.add_marker(skip)
+
+
+@pytest.fixture(autouse=True)
+def the_callers_choice_of_dependent_launches_ends_with_the_test():
+    """A test may switch dependent launches on or off for the whole process (api.set_pdl); the next one runs as users do."""
+    yield
+    from dryft_challenge_htn_2026_b200.csrc import api
+
+    api.set_pdl(None)

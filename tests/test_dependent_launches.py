@@ -97,3 +97,9 @@ def test_a_callers_own_choice_holds_everywhere(libs):
         api.set_pdl(None)
     call("a.cu")
     assert libs["a.cu"].launched[-1] is False
+
+
+@pytest.mark.parametrize("on", [False, True, None])
+def test_what_a_test_chose_does_not_reach_the_next(on):
+    assert api._pdl is None
+    api.set_pdl(on)
