@@ -29,10 +29,10 @@ _pdl = None
 class _Thread(threading.local):
     """What one thread's launches are: inside a model's step or not, and what each library was last told."""
     steps = 0            # model steps this thread is in the middle of
-    dependent = False    # whether the next launch is a dependent one
 
     def __init__(self):
         self.told = {}
+        self.streams = set()     # streams the outermost of those steps has launched something on
 
 
 _thread = _Thread()
@@ -42,8 +42,8 @@ class dependent_launches:
     """``with dependent_launches():`` around the kernels of a model's step. Kernels launched here start under the end of the one
     before them, and some of them read before they wait for it: matrix products their weights, the norms and rotations their
     weights, positions and tables, decode attention its positions, page ids and the cache pages before the newest token's. So
-    nothing launched in here may write any of those. The first launch waits for all that the stream held before, so that the
-    caller may have. Outside, where any call may read what the one before it wrote, every kernel is launched behind the full
+    nothing launched in here may write any of those. The first launch on a stream waits for all that the stream held before, so
+    that the caller may have. Outside, where any call may read what the one before it wrote, every kernel is launched behind the full
     end of the one before. It holds for the calling thread only.
 
     A decode step is a chain of kernels of 2 to 20 us, and pays for every gap between them without. Kernels of a Qwen3 prompt gain
@@ -55,7 +55,7 @@ class dependent_launches:
     def __exit__(self, *exc):
         _thread.steps -= 1
         if _thread.steps == 0:
-            _thread.dependent = False
+            _thread.streams.clear()
 
 
 def set_pdl(on):
@@ -84,7 +84,7 @@ def _lib(source, defines=None):
         lib.dk_set_pdl(int(bool(_pdl)))
         lib.dk_error_string.restype = ctypes.c_char_p
     thread = _thread
-    want = thread.dependent if _pdl is None else _pdl
+    want = (thread.steps > 0 and _stream_ptr() in thread.streams) if _pdl is None else _pdl
     if thread.told.get(key) is not want:
         lib.dk_set_thread_pdl(int(want))
         thread.told[key] = want
@@ -116,7 +116,7 @@ def _check(lib, err, what, kernels=1):
     global _launches
     _launches += kernels
     if _thread.steps:
-        _thread.dependent = True
+        _thread.streams.add(_stream_ptr())
     if err != 0:
         msg = lib.dk_error_string(err).decode()
         raise KernelError(f"{what}: CUDA error {err} ({msg})")

@@ -37,6 +37,7 @@ class Library:
 def libs(monkeypatch):
     found = {"a.cu": Library(), "b.cu": Library()}
     monkeypatch.setattr(api, "_cuda_seen", True)
+    monkeypatch.setattr(api, "_stream_ptr", lambda: 0)
     monkeypatch.setattr(build, "load_lib", lambda source, defines=None: build._libs.setdefault(
         (source, tuple(sorted((defines or {}).items()))), found[source]))
     yield found
@@ -74,6 +75,16 @@ def test_a_step_starts_whole_and_goes_on_dependent(libs):
             1 / 0
     call("a.cu")
     assert libs["a.cu"].launched[3:] == [False, True, False]
+
+
+def test_a_second_stream_within_a_step_starts_whole_as_well(libs, monkeypatch):
+    on = [0]
+    monkeypatch.setattr(api, "_stream_ptr", lambda: on[0])
+    for _ in range(2):
+        with api.dependent_launches():
+            for on[0] in (0, 0, 7, 7, 0, 7):
+                call("a.cu")
+    assert libs["a.cu"].launched == [False, True, False, True, True, True] * 2
 
 
 def test_another_threads_calls_are_not_part_of_the_step(libs):
