@@ -396,7 +396,7 @@ static int launch_gla_warp(const void* q, const void* k, const void* v, long lon
     const dim3 grid(n_seq, nh, (hdv + 31) / 32), block(128);
 #define GLA_WARP(D)                                                                                                    \
     if (hd == 32 * D)                                                                                                  \
-        return dk_launch(gla_warp_kernel<T, D>, grid, block, 0, st, (const T*)q, (const T*)k, (const T*)v, ld, alpha, out, \
+        return dk_launch_as(pdl_on() && cu_q == nullptr, gla_warp_kernel<T, D>, grid, block, 0, st, (const T*)q, (const T*)k, (const T*)v, ld, alpha, out, \
                          state, cu_q, seq_pos0, seq_slot, nh, hdv, q_scale, vec);
     if (vec && n_tok_max > 4) {      // portions: staged rows (single tokens have nothing to run ahead of)
         // columns a warp and a block: coarse when the sequences and heads alone fill the schedulers, finer when not
@@ -415,7 +415,7 @@ static int launch_gla_warp(const void* q, const void* k, const void* v, long lon
         const size_t smem = n_stages * stage;                                                                              \
         if (smem > 48 * 1024)                                                                                              \
             cudaFuncSetAttribute(gla_warp_staged_kernel<T, D, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-        return dk_launch(gla_warp_staged_kernel<T, D, V>, sgrid, sblock, smem, st, (const T*)q, (const T*)k, (const T*)v,  \
+        return dk_launch_whole(gla_warp_staged_kernel<T, D, V>, sgrid, sblock, smem, st, (const T*)q, (const T*)k, (const T*)v,  \
                          ld, alpha, out, state, cu_q, seq_pos0, seq_slot, nh, hdv, q_scale, BC, n_stages);                 \
     }
         GLA_STAGED(1, 8) GLA_STAGED(2, 8) GLA_STAGED(4, 8) GLA_STAGED(8, 8)
@@ -504,7 +504,7 @@ static int launch_step(const void* q, const void* k, const void* v, long long ld
     if (ept <= E) {                                                                                                      \
         if (smem > 48 * 1024)                                                                                            \
             cudaFuncSetAttribute(linear_attention_step_kernel<T, E, GATED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-        return dk_launch(linear_attention_step_kernel<T, E, GATED>, grid, block, smem, st, (const T*)q, (const T*)k, (const T*)v, \
+        return dk_launch_as(pdl_on() && cu_q == nullptr, linear_attention_step_kernel<T, E, GATED>, grid, block, smem, st, (const T*)q, (const T*)k, (const T*)v, \
                          ld, out, state, cu_q, seq_pos0, seq_slot, decay, nh, hd, hdv, cols_pad, cslice, zrows, zbias,    \
                          inv_tau, q_scale);                                                                              \
     }

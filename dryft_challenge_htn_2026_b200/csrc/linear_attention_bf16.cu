@@ -282,7 +282,7 @@ static int launch_chunk(const void* q, const void* k, const void* v, long long l
         cudaFuncSetAttribute(linear_attention_chunk_kernel<DVB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         attr = true;
     }
-    return dk_launch(linear_attention_chunk_kernel<DVB>, dim3(n_seq, nh, hdv / DVB), dim3(LC_THREADS), smem, st, (const bf16*)q,
+    return dk_launch_whole(linear_attention_chunk_kernel<DVB>, dim3(n_seq, nh, hdv / DVB), dim3(LC_THREADS), smem, st, (const bf16*)q,
                      (const bf16*)k, (const bf16*)v, ld, out, state, cu_q, seq_slot, decay, nh, hdv);
 }
 

@@ -477,7 +477,7 @@ static int launch_portion(const void* q, const void* k, const void* v, long long
         const size_t smem = n_stages * stage;                                                                                  \
         if (smem > 48 * 1024)                                                                                                  \
             cudaFuncSetAttribute(mm_portion_kernel<T, D, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);          \
-        return dk_launch(mm_portion_kernel<T, D, V>, grid, block, smem, st, (const T*)q, (const T*)k, (const T*)v, ld,         \
+        return dk_launch_whole(mm_portion_kernel<T, D, V>, grid, block, smem, st, (const T*)q, (const T*)k, (const T*)v, ld,         \
                          (float4*)scal, out, state, n_state, cu_q, seq_pos0, seq_slot, nh, hd, hdv, q_scale, BC, n_stages, vec); \
     }
     MM_GO(1, 8) MM_GO(2, 8) MM_GO(4, 8) MM_GO(8, 8)

@@ -232,9 +232,9 @@ DK_EXPORT int dk_recurrence(const float* q, const float* k, const float* v, long
 #define REC_LAUNCH(D)                                                                                                        \
     if (hd <= 32 * D) {                                                                                                      \
         if (vec)                                                                                                             \
-            return dk_launch(recurrence_kernel<D, true>, grid, block, 0, st, q, k, v, ld, a, out, state, cu_q, seq_pos0, seq_slot, \
+            return dk_launch_as(pdl_on() && cu_q == nullptr, recurrence_kernel<D, true>, grid, block, 0, st, q, k, v, ld, a, out, state, cu_q, seq_pos0, seq_slot, \
                              nh, hd, hdv);                                                                                   \
-        return dk_launch(recurrence_kernel<D, false>, grid, block, 0, st, q, k, v, ld, a, out, state, cu_q, seq_pos0, seq_slot, nh, \
+        return dk_launch_as(pdl_on() && cu_q == nullptr, recurrence_kernel<D, false>, grid, block, 0, st, q, k, v, ld, a, out, state, cu_q, seq_pos0, seq_slot, nh, \
                          hd, hdv);                                                                                           \
     }
     REC_LAUNCH(1) REC_LAUNCH(2) REC_LAUNCH(3) REC_LAUNCH(4) REC_LAUNCH(6) REC_LAUNCH(8)
