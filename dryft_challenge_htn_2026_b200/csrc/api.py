@@ -599,13 +599,13 @@ STREAM_SMALL_WEIGHTS = 8 << 20              # numbers of a matrix below which fe
 
 @functools.lru_cache(maxsize=4096)
 def few_rows_plan(M, N, K, mode, allow_partial=False):
-    """(the streaming product's plan for up to STREAM_BEST_ROWS rows, whether its sums leave as a single float32 part), or (None, False) where the tensor-core product in its decode form
-    (``skinny_tc_plan``) is the faster one: products that may stay in parts and are at least as deep as wide (a layer's output
+    """(the streaming product's plan for up to STREAM_BEST_ROWS rows, whether its sums leave as a single float32 part), or (None,
+    False) where the tensor-core product in its decode form (``skinny_tc_plan``) is the faster one: products that may stay in parts and are at least as deep as wide (a layer's output
     and down projections). While whole rows of x fit they stream in one slice with eight warps a block, since every slice costs the
     norm behind it (2,560 outputs of 4,096 at 8 rows, in a chain norm - product: 8.7 us, 9.4 in four slices as two blocks an SM,
     9.6 on the tensor cores; 4,096 of 4,096: 10.2, 11.0, 10.9); deeper ones go to the tensor cores (2,560 of 9,728: 14.9 -> 13.9;
-    4,096 of 12,288: 24.0 -> 22.2; 5,120 of 17,408: 39.0 -> 35.1). Generation with both: one sequence of 4B sizes 69.2 -> 67.0 ms,
-    eight 252 -> 242, three of 8B sizes 98.2 -> 96.0. The gated and the q/k/v product are as fast or faster there alone (21.2 against 22.3
+    4,096 of 12,288: 24.0 -> 22.2; 5,120 of 17,408: 39.0 -> 35.1). Generation with both, 2 to 4 % less: one sequence of
+    4B sizes 69.2 -> 67.0 ms, eight 252 -> 242, three of 8B sizes 98.2 -> 96.0 (on another box 69.2, 250 and 98 with both). The gated and the q/k/v product are as fast or faster there alone (21.2 against 22.3
     us, 8.9 against 9.1), but whole generations were 1 to 4 % slower with them on the tensor cores: their blocks take an SM's whole
     shared memory, which the attention and rotation between them then wait for. Small matrices stay with ``stream_plan``. Where it would
     have cut a product into slices, whose sums go on in float32, the one slice that takes their place goes on in float32 too."""
@@ -746,7 +746,7 @@ def skinny_tc_plan(M, N, K, mode, allow_partial=False):
     a slice (x waves, should the tiles alone exceed the SMs). The plan with the smallest such unit
     wins; among plans within 3 % of it the one with the fewest slices (partial sums are written and
     added up again), then the larger tile. Slices hold at least 8 blocks of 64 columns (fewer
-    cannot keep the load ring busy). The gated product has no slices (SiLU needs whole sums)."""
+    cannot keep the load ring busy; 6 up to 32 rows, where ``_few_units_plan`` plans). The gated product has no slices (SiLU needs whole sums)."""
     kb = (K + 63) // 64
     sms = sm_count()
     if mode == MODE_SILU:
@@ -776,7 +776,7 @@ def skinny_tc_plan(M, N, K, mode, allow_partial=False):
 
 
 def _few_units_plan(N, kb, sms):
-    """skinny_tc_plan up to 32 rows: units for at most nine tenths of the SMs, the tallest tiles among equals. From about 136
+    """skinny_tc_plan up to 32 rows: units for at most nine tenths of the SMs, the lowest tiles among equals. From about 136
     units of 148 on the chain norm - product - norm takes 1 to 2 us longer (16 rows, 4,096 outputs of 4,096: 145 units 14.1 us, 130
     units of the same length 12.4), since the short kernels around it find no SM of their own; and a block of K costs a unit
     about as much as 40 more weight rows, a slice as much as 50 rows. Against the smallest unit on all SMs (us at 16 rows): 6,144

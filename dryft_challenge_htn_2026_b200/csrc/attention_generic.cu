@@ -1,5 +1,6 @@
 // Causal grouped-query attention over the paged cache, one warp per (token, query head), all
-// arithmetic in float32 on CUDA cores. It serves the 32-bit path of the model for every phase
+// arithmetic in float32 on CUDA cores. It serves the 32-bit path of the model where attention_f32.cu does not
+// (head sizes other than 64 and 128, more than 16 query heads a kv head), in every phase
 // (whole prompts, continued chunks, single tokens); any head size that is a multiple of 2 up to
 // 256, any head counts, an optional sliding window.
 //

@@ -22,7 +22,8 @@ def linear(x, w, mode=STORE, allow_partial=False, act=(0.0, 0.0)):
     (alpha_pos, alpha_neg), in the product's epilogue wherever the product is this library's (after
     the library's product a row kernel applies it). ``allow_partial``: the caller can take
     ``csrc.api.Partial`` (split-K partial sums, added up by the kernel that consumes them) instead
-    of a tensor (with STORE_F32 too: partial sums are float32)."""
+    of a tensor (with STORE_F32 too: partial sums are float32). Within a model's step ``w`` is read before the kernel in front of
+    the product has ended (``csrc.api.dependent_launches``): nothing of the step may write it."""
     M, K = x.shape
     N = w.shape[0] // 2 if mode == SILU else w.shape[0]
     if x.dtype == torch.float32:
