@@ -422,7 +422,9 @@ F32_TC_MIN_K = 256
 F32_CHUNK = 64              # columns of K that gemm_f32_tc adds up in tensor memory at a time
 F32_MAX_ROW_TILE = 128      # rows of x a tile
 F32_PIECES_BYTES = 256 << 20  # most scratch memory for the pieces of x; more rows go in several launches
-F32_TILE_HEIGHTS = (128, 112, 96, 80, 64, 56, 48, 40, 32)      # outputs a tile (the gated product: half of them)
+F32_TILE_HEIGHTS = (128, 120, 112, 96, 80, 64, 56, 48, 40, 32)      # outputs a tile (the gated product: half of them)
+F32_DIRECT_ROWS = 4         # up to so many rows of x the product takes apart itself, in row tiles of at most F32_FEW_ROW_TILE
+F32_FEW_ROW_TILE = 32
 
 
 def f32_groups(N, K, mode=MODE_STORE):
@@ -441,9 +443,12 @@ def f32_groups(N, K, mode=MODE_STORE):
 def f32_plan(M, N, K, mode=MODE_STORE, allow_partial=False):
     """(outputs a tile, rows of x a tile, split) for gemm_f32_tc; ``split``: a unit of work takes one group of K and leaves
     partial sums. The plan with the least modelled time wins: waves of units x clocks of a unit. A chunk of 64 columns
-    takes the longest of its 24 mma (half a clock a row, at least 50) and its bytes (of weights at a 148th of the HBM rate, 24 a
-    clock; of weights and pieces of x at 40 a clock from the L2); a unit 2,500 more to fill and drain. Partial sums are written and read again at
-    the same rate; adding a group into ``out`` costs a unit about 1,500."""
+    takes the longest of its 24 mma (half a clock a row and 8, 150 a chunk between them), its conversion (1,150 measured where the
+    mma are short: one row of 9,728 gated outputs takes 50 to 52 us with tiles of 28 to 16 outputs) and its bytes (of weights at a
+    148th of the HBM rate, 24 a clock; of weights and pieces of x at 55 a clock from the L2); a unit 2,500 more to fill and drain.
+    Partial sums are read by their consumer at the same rate; adding a group into ``out`` costs a unit about 4,000 (544 rows, 2,560
+    outputs of 4,096: 97 us with groups added, 71 in parts). Sweeps of all plans at 1 to 1,000 rows of the 4B widths: what this
+    picks is within 3 % of the best."""
     sms = sm_count()
     kb = (K + F32_CHUNK - 1) // F32_CHUNK
     groups, length = f32_groups(N, K, mode)
@@ -457,12 +462,12 @@ def f32_plan(M, N, K, mode=MODE_STORE, allow_partial=False):
         for height in F32_TILE_HEIGHTS:
             tile_n = height // per_out
             bytes_w = per_out * tile_n * 256
-            chunk = max(24 * max(nt / 2, 50), bytes_w / 24 / row_tiles, (bytes_w + 384 * nt) / 40)
+            chunk = max(24 * (nt / 2 + 8) + 150, 1150, bytes_w / 24 / row_tiles, (bytes_w + 384 * nt) / 55)
             tiles = (N + tile_n - 1) // tile_n
             for split in ((False, True) if allow_partial and groups > 1 and f32_rows_a_launch(M, K) == M else (False,)):
                 units = tiles * row_tiles * (groups if split else 1)
-                unit = (length if split else kb) * chunk + 2500 + (0 if split else (groups - 1) * 1500)
-                cost = -(-units // sms) * unit + (groups * M * N * 8 / (sms * 24) if split else 0)
+                unit = (length if split else kb) * chunk + 2500 + (0 if split else (groups - 1) * 4000)
+                cost = -(-units // sms) * unit + (groups * M * N * 4 / (sms * 24) if split else 0)
                 if best is None or cost < best[0]:
                     best = cost, (tile_n, nt, split)
     return best[1]
@@ -501,7 +506,8 @@ def gemm_f32_tc(x, w, mode=MODE_STORE, plan=None, act=(0.0, 0.0), out=None):
     if M == 0:
         return out
     rows = M if split else f32_rows_a_launch(M, K)
-    pieces = torch.empty(3 * rows * ((K + 7) // 8 * 8), dtype=torch.bfloat16, device=x.device)
+    direct = M <= F32_DIRECT_ROWS and nt <= F32_FEW_ROW_TILE
+    pieces = None if direct else torch.empty(3 * rows * ((K + 7) // 8 * 8), dtype=torch.bfloat16, device=x.device)
     if _tc_err is None:
         _tc_err = torch.zeros(1, dtype=torch.int32, device=x.device)
     lib = _lib("gemm_f32_tc.cu")
@@ -509,7 +515,7 @@ def gemm_f32_tc(x, w, mode=MODE_STORE, plan=None, act=(0.0, 0.0), out=None):
         _check(lib, lib.dk_gemm_f32_tc(c_void_p(x.data_ptr() + 4 * m * K), _p(w), c_void_p(0 if split else out.data_ptr() + 4 * m * N),
                                        _p(pieces), min(rows, M - m), N, K, 0 if mode == MODE_STORE_F32 else mode,
                                        groups, length, _p(ws), tile_n, nt, _p(_tc_err), c_float(act[0]), c_float(act[1]),
-                                       _stream()), "gemm_f32_tc", 2)
+                                       _stream()), "gemm_f32_tc", 1 if direct else 2)
     return Partial(ws) if split else out
 
 

@@ -18,19 +18,23 @@
 // Where a unit of work holds one group (split) the groups leave as partial sums [S][M][N] for the consumer to add
 // up in the same order; where it holds all of them (few units otherwise) it adds group after group into ``out`` itself.
 //
-// What bounds it: few rows: the weights' bytes from HBM (a ring of 2 to 5 stages of 32 KB an SM); many rows: the six
-// products, one sixth of the bfloat16 rate. Roles of a block (one per SM, persistent over units):
-//   warps 0-7   convert: two threads take row r of a stage's weights (128 rows x 64 columns, float32, TMA with 128-byte
-//               swizzle), 32 columns each, and write its three bfloat16 pieces into tensor memory, where the mma reads its
-//               A operand from (96 columns a stage, two stages). In shared memory the pieces would cost 48 KB a stage
-//               written, and the mma 8 instead of 4 KB read per 128 x 128 x 16 product.
-//   warps 8-15  drain: two threads a row, half of the columns each, add up the two accumulators in turn; epilogue.
-//   warp 16     TMA of the weights; warp 17 tcgen05.mma; warp 18 TMA of the pieces of x ([3][M][Kp] bfloat16, made by
-//               split_rows before: as the B operand they come ready from shared memory).
-// Measured in a graph (2,560 wide layers of 9,728; sgemm -> this kernel with split_rows): 544 rows: q/k/v 740 -> 113 us, output
-// projection 609 -> 97, gated 1,994 -> 349, down 1,455 -> 163 (165 TFLOP/s; without the mma the gated product takes 231: the
-// tiles' 75 KB a chunk from the L2 and the mma overlap in part only). One row: 175 -> 14, 273 -> 11, 409 -> 57, 839 -> 19, a
-// head of 151,936 1,733 -> 260 (6.0 TB/s).
+// What bounds it: few rows: the weights' bytes from HBM while all SMs have a unit, then the chunks of the units left (about 1,150
+// clocks each, whatever their height); many rows: the six products, one sixth of the bfloat16 rate, under the power cap.
+// Roles of a block (one per SM, persistent over units), in two forms: tiles of more than 32 rows of x, and FEW:
+//   convert (8 warps; FEW 16 in two groups that take chunks in turn): two threads take row r of a stage's weights (up to 128 rows x
+//               64 columns, float32, TMA with 128-byte swizzle), 32 columns each, and write its three bfloat16 pieces into tensor
+//               memory, where the mma reads its A operand from (96 columns a buffer, 2 to 4 buffers). In shared memory the pieces
+//               would cost 48 KB a stage written, and the mma 8 instead of 4 KB read per 128 x 128 x 16 product. One group alone
+//               takes 1,250 clocks a chunk with loads, arithmetic and stores one after the other.
+//   drain (8 warps, two threads a row, half of the columns each; FEW 4, one thread a row): adds up the accumulators in turn; epilogue.
+//   a warp for the TMA of the weights, one for x, two that issue tcgen05.mma: they take chunks in turn, so that the three waits of a
+//               chunk (250 to 350 clocks together) run beside the mma of the other one's.
+//   x: FEW and at most 4 rows: the warp loads them as float32 and takes them apart itself, two chunks ahead; else TMA of the pieces
+//               ([3][M][Kp] bfloat16, made by split_rows before: as the B operand they come ready from shared memory).
+// Measured in a graph (2,560 wide layers of 9,728; one converting group, one mma warp, descriptors built at each mma and split_rows in
+// front of every product -> this kernel; sgemm before both): one row: q/k/v 16.4 -> 12.4 us, output projection 13.8 -> 9.6, gated
+// 60.9 -> 50.1, down 22.1 -> 18.0 (the weights' bytes take 9.6, 6.4, 30.5, 15.2), a head of 50,000 91 -> 82 (6.2 TB/s). 544 rows:
+// 118 -> 99, 112 -> 71, 354 -> 332, 166 -> 156.
 // Infinities, NaN and numbers beyond bfloat16's largest: a piece times a zero piece is NaN where the product is not. A
 // thread that finds a sum that is not finite works that one out again by plain FMA from x and W.
 #include <cuda.h>
@@ -39,10 +43,10 @@
 
 namespace {
 
-constexpr int BK = 64, ROWS = 128, MAX_NT = 128, MAX_STAGES = 6;
-constexpr int HALF_BYTES = ROWS * 128, W_STAGE = 2 * HALF_BYTES;      // 128 rows x 32 floats, twice
-constexpr int A_COLS = 96, A_BASE = 2 * MAX_NT;
-constexpr int EX_BYTES = 2 * 32 * 64 * 4, HALF_COLS = MAX_NT / 2;
+constexpr int BK = 64, ROWS = 128, MAX_NT = 128, MAX_STAGES = 12, MAX_BUFS = 4;
+constexpr int A_COLS = 96;
+constexpr int DIRECT_ROWS = 4;                    // up to so many rows of x are taken apart by the product itself
+constexpr int EX_BYTES = 2 * 32 * 64 * 4, FEW_NT = 32;   // up to FEW_NT rows a tile: the kernel's form for few rows
 #ifndef DK_WAIT_CYCLES
 #define DK_WAIT_CYCLES 2000000000LL               // about a second: a wait this long has failed
 #endif
@@ -209,7 +213,7 @@ struct Product {
     float *out, *parts;          // parts: [S][M][N] where a unit holds one group
     int M, N, K, Kp;
     int tile_n, tiles, nt, row_tiles, groups, group_len, split;   // tile_n: outputs a tile (weight rows; mode 2: half of them)
-    int w_stages, x_stages;
+    int w_stages, x_stages, w_box, bufs;   // w_box: bytes between boxes of weights in shared memory; bufs: pieces of W, accumulators
     float act_pos, act_neg;
 };
 
@@ -227,20 +231,29 @@ __device__ __noinline__ float plain_sum(const float* x, const float* w, int K, i
     return total;
 }
 
-template <int MODE>
-__global__ void __launch_bounds__(608, 1)
+// FEW (tiles of at most FEW_NT rows): 16 converting warps in two groups that take chunks in turn, and 4 draining ones; else 8 and 8.
+template <bool FEW>
+struct Warps {
+    static constexpr int CONVERT = FEW ? 16 : 8, DRAIN = FEW ? 4 : 8, LOADER = CONVERT + DRAIN, THREADS = (LOADER + 4) * 32;
+};
+
+template <int MODE, bool FEW>
+__global__ void __launch_bounds__(Warps<FEW>::THREADS, 1)
 gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
                    const __grid_constant__ Product p, int* err) {
+    constexpr int CONVERT = Warps<FEW>::CONVERT, DRAIN = Warps<FEW>::DRAIN, LOADER = Warps<FEW>::LOADER;
+    constexpr int HALF_COLS = FEW ? FEW_NT : MAX_NT / 2;      // columns a draining thread adds up: all, or half of them
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);
     const int x_piece = p.nt * 128, x_stage = 3 * x_piece;
+    const int w_half = (MODE == 2 ? 2 : 1) * p.w_box, w_stage = 2 * w_half;   // rows x 32 floats (mode 2: gate rows, up rows), twice
     uint8_t* smem_w = smem;
-    uint8_t* smem_x = smem_w + p.w_stages * W_STAGE;
+    uint8_t* smem_x = smem_w + p.w_stages * w_stage;
     float* exchange = reinterpret_cast<float*>(smem_x + p.x_stages * x_stage);          // mode 2: [2][32][64] up sums
     uint64_t* w_full = reinterpret_cast<uint64_t*>(reinterpret_cast<uint8_t*>(exchange) + EX_BYTES);
     uint64_t *w_empty = w_full + MAX_STAGES, *x_full = w_empty + MAX_STAGES, *x_empty = x_full + MAX_STAGES;
-    uint64_t *a_full = x_empty + MAX_STAGES, *a_empty = a_full + 2, *acc_full = a_empty + 2, *acc_empty = acc_full + 2;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+    uint64_t *a_full = x_empty + MAX_STAGES, *a_empty = a_full + MAX_BUFS, *acc_full = a_empty + MAX_BUFS, *acc_empty = acc_full + MAX_BUFS;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + MAX_BUFS);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int k_blocks = (p.K + BK - 1) / BK;
     const int slices = p.split ? p.groups : 1, per = p.split ? p.group_len : k_blocks;
@@ -256,14 +269,14 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
             mbar_init(&w_full[s], 1), mbar_init(&w_empty[s], 8);
             mbar_init(&x_full[s], 1), mbar_init(&x_empty[s], 1);
         }
-        for (int b = 0; b < 2; b++) {
+        for (int b = 0; b < MAX_BUFS; b++) {
             mbar_init(&a_full[b], 8), mbar_init(&a_empty[b], 1);
-            mbar_init(&acc_full[b], 1), mbar_init(&acc_empty[b], 8);
+            mbar_init(&acc_full[b], 1), mbar_init(&acc_empty[b], DRAIN);
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
-    if (warp == 17) {
+    if (warp == LOADER + 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -271,9 +284,9 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem = *tmem_slot;
+    const uint32_t tmem = *tmem_slot, a_base = tmem + p.bufs * p.nt;   // accumulators of nt columns, then the pieces of W
 
-    if (warp == 16) {
+    if (warp == LOADER) {
         if (lane == 0) {  // ------------------------------------ weights (no kernel of a step writes them)
             const uint64_t stream_once = l2_evict_first();
             const uint32_t tx = (MODE == 2 ? 2 : 1) * p.tile_n * 256;
@@ -288,23 +301,82 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
                         ok = false;
                         break;
                     }
-                    uint8_t* stage = smem_w + s * W_STAGE;
+                    uint8_t* stage = smem_w + s * w_stage;
                     mbar_expect_tx(&w_full[s], tx);
                     for (int h = 0; h < 2; h++) {
                         if (p.row_tiles == 1) {
-                            tma_load_2d(stage + h * HALF_BYTES, &map_w, kb * BK + 32 * h, n0, &w_full[s], stream_once);
+                            tma_load_2d(stage + h * w_half, &map_w, kb * BK + 32 * h, n0, &w_full[s], stream_once);
                             if (MODE == 2)
-                                tma_load_2d(stage + h * HALF_BYTES + 64 * 128, &map_w, kb * BK + 32 * h, p.N + n0, &w_full[s], stream_once);
+                                tma_load_2d(stage + h * w_half + p.w_box, &map_w, kb * BK + 32 * h, p.N + n0, &w_full[s], stream_once);
                         } else {
-                            tma_load_2d(stage + h * HALF_BYTES, &map_w, kb * BK + 32 * h, n0, &w_full[s]);
+                            tma_load_2d(stage + h * w_half, &map_w, kb * BK + 32 * h, n0, &w_full[s]);
                             if (MODE == 2)
-                                tma_load_2d(stage + h * HALF_BYTES + 64 * 128, &map_w, kb * BK + 32 * h, p.N + n0, &w_full[s]);
+                                tma_load_2d(stage + h * w_half + p.w_box, &map_w, kb * BK + 32 * h, p.N + n0, &w_full[s]);
                         }
                     }
                 }
             }
         }
-    } else if (warp == 18) {
+    } else if (FEW && warp == LOADER + 2 && p.M <= DIRECT_ROWS) {  // ----------- few rows of x: taken apart here
+        pdl_wait();
+        if (lane == 0) pdl_launch_dependents();
+        const bool aligned = (reinterpret_cast<uintptr_t>(p.x) & 15) == 0;
+        const int row = lane >> 3;
+        int s = 0, it = 0;
+        uint32_t round = 0;
+        bool ok = true;
+        for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
+            UNIT(u);
+            float va[2][8], vb[2][8];                         // two chunks at a time, the next two on their way
+            auto load = [&](float (&v)[2][8], int kb) {
+#pragma unroll
+                for (int j = 0; j < 2; j++)                   // a lane takes 8 columns of row lane / 8
+#pragma unroll
+                    for (int e = 0; e < 8; e += 4) {          // K is a multiple of 4; zeros behind it
+                        const int k = (kb + j) * BK + (lane & 7) * 8 + e;
+                        float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
+                        if (row < p.M && kb + j < kb1 && k < p.K) {
+                            const float* src = p.x + (size_t)row * p.K + k;
+                            if (aligned) f = *reinterpret_cast<const float4*>(src);
+                            else f = make_float4(src[0], src[1], src[2], src[3]);
+                        }
+                        v[j][e] = f.x, v[j][e + 1] = f.y, v[j][e + 2] = f.z, v[j][e + 3] = f.w;
+                    }
+            };
+            auto put = [&](const float (&v)[2][8], int kb) {
+#pragma unroll
+                for (int j = 0; j < 2; j++) {
+                    if (kb + j >= kb1 || !ok) continue;
+                    if (it >= p.x_stages) ok = __all_sync(0xffffffffu, mbar_wait(&x_empty[s], round ^ 1));
+                    if (!ok) {
+                        atomicExch(err, 12);
+                        continue;
+                    }
+                    if (row < p.M) {                          // rows behind M hold anything: their sums are never stored
+                        uint32_t h[4], m[4], l[4];
+#pragma unroll
+                        for (int e = 0; e < 4; e++) split_pair(v[j][2 * e], v[j][2 * e + 1], h[e], m[e], l[e]);
+                        uint8_t* to = smem_x + s * x_stage + row * 128 + (((lane & 7) ^ (row & 7)) << 4);
+                        *reinterpret_cast<uint4*>(to) = make_uint4(h[0], h[1], h[2], h[3]);
+                        *reinterpret_cast<uint4*>(to + x_piece) = make_uint4(m[0], m[1], m[2], m[3]);
+                        *reinterpret_cast<uint4*>(to + 2 * x_piece) = make_uint4(l[0], l[1], l[2], l[3]);
+                    }
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&x_full[s]);
+                    it++;
+                    if (++s == p.x_stages) s = 0, round ^= 1;
+                }
+            };
+            load(va, kb0);
+            for (int kb = kb0; kb < kb1 && ok; kb += 4) {
+                load(vb, kb + 2);
+                put(va, kb);
+                load(va, kb + 4);
+                put(vb, kb + 2);
+            }
+        }
+    } else if (warp == LOADER + 2) {
         if (lane == 0) {  // ------------------------------------ the pieces of x
             pdl_wait();
             pdl_launch_dependents();
@@ -325,19 +397,23 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
                 }
             }
         }
-    } else if (warp == 17) {
-        // ---------------------------------------------------------------------- mma
+    } else if (warp == LOADER + 1 || warp == LOADER + 3) {
+        // ------------------------ mma: two warps take chunks in turn, so that the waits of one run beside the mma of the other
+        const int mine = warp == LOADER + 3;
         const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(p.nt >> 3) << 17) | ((uint32_t)(ROWS >> 4) << 24);
-        int xs = 0, it = 0;
-        uint32_t xround = 0;
+        int xs = 0, it = 0, b = 0;
+        uint32_t xround = 0, phase = 0;
+        // a piece further on in shared memory is an addition to the low half of the descriptor (in units of 16 bytes)
+        const uint64_t x_desc = umma_desc(smem_u32(smem_x));
+        const uint32_t piece = (uint32_t)x_piece >> 4;
         bool ok = true;
         for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
             UNIT(u);
-            for (int kb = kb0; kb < kb1; kb++, it++, xs = xs + 1 == p.x_stages ? 0 : xs + 1, xround ^= (xs == 0)) {
-                const int b = it & 1;
-                const uint32_t phase = (it >> 1) & 1;
+            for (int kb = kb0; kb < kb1; kb++, it++, xs = xs + 1 == p.x_stages ? 0 : xs + 1, xround ^= (xs == 0),
+                     b = b + 1 == p.bufs ? 0 : b + 1, phase ^= (b == 0)) {
+                if ((it & 1) != mine) continue;
                 ok = mbar_wait(&x_full[xs], xround) && mbar_wait(&a_full[b], phase) &&
-                     (it < 2 || mbar_wait(&acc_empty[b], phase ^ 1));
+                     (it < p.bufs || mbar_wait(&acc_empty[b], phase ^ 1));
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) {
                     atomicExch(err, 13);
@@ -345,8 +421,8 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 if (elect_one()) {
-                    const uint32_t d = tmem + b * MAX_NT, a = tmem + A_BASE + b * A_COLS;
-                    const uint32_t xb = smem_u32(smem_x + xs * x_stage);
+                    const uint32_t d = tmem + b * p.nt, a = a_base + b * A_COLS;
+                    const uint64_t xb = x_desc + (uint32_t)(xs * 3) * piece, x_at[3] = {xb, xb + piece, xb + 2 * piece};
                     // (piece of W, piece of x), 0 the largest; the products grow from the first to the last, at 2^16, 2^8 and 1
                     constexpr int PA[6] = {2, 0, 1, 1, 0, 0}, PB[6] = {0, 2, 1, 0, 1, 0};
 #pragma unroll
@@ -354,7 +430,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
 #pragma unroll
                         for (int k = 0; k < BK / 16; k++) {
                             const uint32_t ak = a + PA[q] * 32 + k * 8;
-                            const uint64_t bk = umma_desc(xb + PB[q] * x_piece + k * 32);
+                            const uint64_t bk = x_at[PB[q]] + 2 * k;
                             if (k == 0 && q > 0 && PA[q] + PB[q] < PA[q - 1] + PB[q - 1]) umma_ts_down8(d, ak, bk, idesc);
                             else umma_ts(d, ak, bk, idesc, (q | k) != 0);
                         }
@@ -365,35 +441,42 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
                 __syncwarp();
             }
         }
-    } else if (warp < 8) {  // -------------------------------------------------- convert
-        const int r = threadIdx.x & 127, h = warp >> 2;
-        const uint32_t to = tmem + A_BASE + h * 16 + ((uint32_t)((warp & 3) * 32) << 16);
-        int ws = 0, it = 0;
-        uint32_t wround = 0;
+    } else if (warp < CONVERT) {  // -------------------------------------------------- convert
+        const int r = threadIdx.x & 127, h = (warp >> 2) & 1, group = warp >> 3;
+        const uint32_t to = a_base + h * 16 + ((uint32_t)((warp & 3) * 32) << 16);
+        // where row r of a half stage lies; lanes without a row of the tile read the first one's, and their sums are never stored
+        const int in_tile = MODE == 2 ? r & 63 : r;
+        const int place = in_tile < p.tile_n ? (MODE == 2 ? (r >> 6) * p.w_box : 0) + in_tile * 128 : 0, turn = (place >> 7) & 7;
+        const bool idle = (MODE == 2 ? (warp & 1) * 32 : (warp & 3) * 32) >= p.tile_n;     // no lane of the warp has one
+        int ws = 0, it = 0, b = 0;
+        uint32_t wround = 0, phase = 0;
         bool ok = true;
         for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
             UNIT(u);
-            for (int kb = kb0; kb < kb1; kb++, it++, ws = ws + 1 == p.w_stages ? 0 : ws + 1, wround ^= (ws == 0)) {
-                const int b = it & 1;
+            for (int kb = kb0; kb < kb1; kb++, it++, ws = ws + 1 == p.w_stages ? 0 : ws + 1, wround ^= (ws == 0),
+                     b = b + 1 == p.bufs ? 0 : b + 1, phase ^= (b == 0)) {
+                if (FEW && (it & 1) != group) continue;
                 ok = mbar_wait(&w_full[ws], wround);
-                if (ok && it >= 2) ok = mbar_wait(&a_empty[b], ((it >> 1) & 1) ^ 1);
+                if (ok && it >= p.bufs) ok = mbar_wait(&a_empty[b], phase ^ 1);
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) {
                     atomicExch(err, 14);
                     break;
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint8_t* row = smem_w + ws * W_STAGE + h * HALF_BYTES + r * 128;
-                uint32_t hi[16], mid[16], lo[16];
+                if (!idle) {
+                    const uint8_t* row = smem_w + ws * w_stage + h * w_half + place;
+                    uint32_t hi[16], mid[16], lo[16];
 #pragma unroll
-                for (int c = 0; c < 8; c++) {
-                    const float4 v = *reinterpret_cast<const float4*>(row + ((c ^ (r & 7)) << 4));
-                    split_pair(v.x, v.y, hi[2 * c], mid[2 * c], lo[2 * c]);
-                    split_pair(v.z, v.w, hi[2 * c + 1], mid[2 * c + 1], lo[2 * c + 1]);
+                    for (int c = 0; c < 8; c++) {
+                        const float4 v = *reinterpret_cast<const float4*>(row + ((c ^ turn) << 4));
+                        split_pair(v.x, v.y, hi[2 * c], mid[2 * c], lo[2 * c]);
+                        split_pair(v.z, v.w, hi[2 * c + 1], mid[2 * c + 1], lo[2 * c + 1]);
+                    }
+                    tmem_st16(to + b * A_COLS, hi);
+                    tmem_st16(to + b * A_COLS + 32, mid);
+                    tmem_st16(to + b * A_COLS + 64, lo);
                 }
-                tmem_st16(to + b * A_COLS, hi);
-                tmem_st16(to + b * A_COLS + 32, mid);
-                tmem_st16(to + b * A_COLS + 64, lo);
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&w_empty[ws]);
                 asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
@@ -404,13 +487,14 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
         }
     } else {  // ---------------------------------------------------------------- drain and epilogue
         const int q = warp & 3, r = q * 32 + lane;
-        const int half = (warp - 8) >> 2, split_at = (p.nt / 2 + 15) / 16 * 16;      // columns [0, split_at), [split_at, nt)
+        const int half = FEW ? 0 : (warp - CONVERT) >> 2, split_at = FEW ? p.nt : (p.nt / 2 + 15) / 16 * 16;      // columns [0, split_at), [split_at, nt)
         const int j0 = half * split_at, cols = half ? p.nt - split_at : split_at, pieces = cols / 16;
         float* ex = exchange + half * 32 * 64;
         const bool is_up = MODE == 2 && q >= 2;
         const int local = MODE == 2 ? (r & 63) : r;
         pdl_wait();                       // nothing is stored before the kernels before this one are done
-        int it = 0;
+        int b = 0;
+        uint32_t phase = 0;
         bool ok = true;
         for (int u = blockIdx.x; u < units; u += gridDim.x) {
             UNIT(u);
@@ -423,15 +507,14 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
 #pragma unroll
                 for (int j = 0; j < HALF_COLS; j++) tot[j] = 0.f;
                 const int g1 = min(kb1, g0 + p.group_len);
-                for (int kb = g0; kb < g1; kb++, it++) {
-                    const int b = it & 1;
-                    if (ok) ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[b], (it >> 1) & 1));
+                for (int kb = g0; kb < g1; kb++, b = b + 1 == p.bufs ? 0 : b + 1, phase ^= (b == 0)) {
+                    if (ok) ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[b], phase));
                     if (!ok) {             // go on without waiting: the warps meet at barriers below, and the sums are not valid
                         atomicExch(err, 15);
                         continue;
                     }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint32_t acc = tmem + b * MAX_NT + j0 + ((uint32_t)(q * 32) << 16);
+                    const uint32_t acc = tmem + b * p.nt + j0 + ((uint32_t)(q * 32) << 16);
 #pragma unroll
                     for (int c = 0; c < HALF_COLS / 16; c++)
                         if (c < pieces) {
@@ -506,7 +589,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (warp == 17) {
+    if (warp == LOADER + 1) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
     }
@@ -542,35 +625,49 @@ int make_map(CUtensorMap* map, CUtensorMapDataType type, int size, const void* b
     return r == CUDA_SUCCESS ? 0 : (int)cudaErrorInvalidValue;
 }
 
-template <int MODE>
-int launch(Product p, const bf16* pieces, int* err, cudaStream_t st) {
+template <int MODE, bool FEW>
+int launch_as(Product p, const bf16* pieces, int* err, cudaStream_t st) {
     const int x_stage = 3 * p.nt * 128;
-    const size_t tail = EX_BYTES + (4 * MAX_STAGES + 8) * sizeof(uint64_t) + 16;
+    const size_t tail = EX_BYTES + (4 * MAX_STAGES + 4 * MAX_BUFS) * sizeof(uint64_t) + 16;
     const size_t budget = 227 * 1024 - tail - 1024;
-    // a stage of x is free when its mma are done, a stage of W once it is converted (two more wait in tensor memory)
-    p.x_stages = p.nt > 32 ? 3 : 4;
-    p.w_stages = (int)((budget - (size_t)p.x_stages * x_stage) / W_STAGE);
+    p.w_box = (p.tile_n + 7) / 8 * 1024;                      // 128 bytes a row, boxes at multiples of the swizzle's 1024
+    const int w_stage = (MODE == 2 ? 4 : 2) * p.w_box;
+    p.bufs = 512 / (p.nt + A_COLS) < MAX_BUFS ? 512 / (p.nt + A_COLS) : MAX_BUFS;
+    // a stage of x is free when its mma are done, a stage of W once it is converted (``bufs`` more wait in tensor memory)
+    p.x_stages = p.nt > 64 ? 2 : 4;                           // even: see below
+    p.w_stages = (int)((budget - (size_t)p.x_stages * x_stage) / w_stage);
     if (p.w_stages > MAX_STAGES) p.w_stages = MAX_STAGES;
-    const size_t smem = 1024 + (size_t)p.w_stages * W_STAGE + (size_t)p.x_stages * x_stage + tail;
+    // Warps that take chunks in turn (mma; converting ones, FEW) need an even number of the stages that loads fill, which come in any
+    // order: each then belongs to one of them. A warp that met a stage's barrier only every second time could take the phase before
+    // for its own. (Buffers that warps fill or empty in order may be three.)
+    if (FEW) p.w_stages &= ~1;
+    if (p.w_stages < 1 || (FEW && p.bufs % 2 != 0)) return (int)cudaErrorInvalidValue;
+    const size_t smem = 1024 + (size_t)p.w_stages * w_stage + (size_t)p.x_stages * x_stage + tail;
     int sms = 0, dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaError_t e = cudaFuncSetAttribute(gemm_f32_tc_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    cudaError_t e = cudaFuncSetAttribute(gemm_f32_tc_kernel<MODE, FEW>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     if (e != cudaSuccess) return (int)e;
-    CUtensorMap mx, mw;
-    int rc = make_map(&mx, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, pieces, 3LL * p.M, p.Kp, p.nt);
+    CUtensorMap mx{}, mw;
+    int rc = FEW && p.M <= DIRECT_ROWS ? 0 : make_map(&mx, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, pieces, 3LL * p.M, p.Kp, p.nt);
     if (rc) return rc;
     rc = make_map(&mw, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, p.W, MODE == 2 ? 2LL * p.N : p.N, p.K, p.tile_n);
     if (rc) return rc;
     const long long units = (long long)p.tiles * (p.split ? p.groups : 1) * p.row_tiles;
     if (units > (1LL << 30)) return (int)cudaErrorInvalidValue;
-    return dk_launch(gemm_f32_tc_kernel<MODE>, dim3((unsigned)(units < sms ? units : sms)), dim3(608), smem, st, mx, mw, p, err);
+    return dk_launch(gemm_f32_tc_kernel<MODE, FEW>, dim3((unsigned)(units < sms ? units : sms)), dim3(Warps<FEW>::THREADS), smem, st, mx, mw, p, err);
+}
+
+template <int MODE>
+int launch(const Product& p, const bf16* pieces, int* err, cudaStream_t st) {
+    return p.nt <= FEW_NT ? launch_as<MODE, true>(p, pieces, err, st) : launch_as<MODE, false>(p, pieces, err, st);
 }
 
 }  // namespace
 
 // x [M,K], W [N,K] (mode 2: [2N,K] = gate rows then up rows), out [M,N], all float32; K % 4 == 0, W on a 16-byte boundary.
-// pieces: scratch of 3 * M * Kp bfloat16, Kp = K rounded up to a multiple of 8, on a 16-byte boundary. groups, group_len:
+// pieces: scratch of 3 * M * Kp bfloat16, Kp = K rounded up to a multiple of 8, on a 16-byte boundary (null with at most 4 rows
+// in row tiles of at most 32). groups, group_len:
 // K's chunks of 64 columns in ``groups`` groups of ``group_len`` (the last may be shorter, none empty; 1 in mode 2).
 // parts: null, or [groups][M][N] (mode 0): the groups' sums, left for the consumer to add up. tile_n: outputs a tile, at
 // most 128 (mode 2: 64). nt: rows of x a tile, a multiple of 16, at most 128. err: device int, receives a code if a bounded
@@ -579,16 +676,18 @@ DK_EXPORT int dk_gemm_f32_tc(const float* x, const float* W, float* out, void* p
                              int group_len, float* parts, int tile_n, int nt, int* err, float act_pos, float act_neg,
                              cudaStream_t st) {
     const int k_blocks = (K + BK - 1) / BK, Kp = (K + 7) / 8 * 8;
-    if (M < 1 || N < 1 || K < 4 || K % 4 != 0 || err == nullptr || pieces == nullptr || (mode != 0 && mode != 2 && mode != 3))
+    if (M < 1 || N < 1 || K < 4 || K % 4 != 0 || err == nullptr || (pieces == nullptr && !(M <= DIRECT_ROWS && nt <= FEW_NT)) || (mode != 0 && mode != 2 && mode != 3))
         return (int)cudaErrorInvalidValue;
     if (((uintptr_t)W | (uintptr_t)pieces) % 16 != 0 || 3LL * M > (1LL << 30)) return (int)cudaErrorInvalidValue;
     if (groups < 1 || group_len < 1 || (long long)groups * group_len < k_blocks || (long long)(groups - 1) * group_len >= k_blocks ||
         (mode == 2 && groups != 1) || (parts != nullptr && mode != 0) || (parts == nullptr && out == nullptr))
         return (int)cudaErrorInvalidValue;
     if (tile_n < 1 || tile_n > (mode == 2 ? 64 : 128) || nt < 16 || nt > MAX_NT || nt % 16 != 0) return (int)cudaErrorInvalidValue;
-    const long long threads = (long long)M * (Kp / 8);
-    int e = dk_launch(split_rows_kernel, dim3((unsigned)((threads + 127) / 128)), dim3(128), 0, st, x, (bf16*)pieces, M, K, Kp);
-    if (e) return e;
+    if (M > DIRECT_ROWS || nt > FEW_NT) {
+        const long long threads = (long long)M * (Kp / 8);
+        const int e = dk_launch(split_rows_kernel, dim3((unsigned)((threads + 127) / 128)), dim3(128), 0, st, x, (bf16*)pieces, M, K, Kp);
+        if (e) return e;
+    }
     Product p{};
     p.x = x, p.W = W, p.out = out, p.parts = parts, p.M = M, p.N = N, p.K = K, p.Kp = Kp;
     p.tile_n = tile_n, p.tiles = (N + tile_n - 1) / tile_n, p.nt = nt, p.row_tiles = (M + nt - 1) / nt;

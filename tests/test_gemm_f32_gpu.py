@@ -116,3 +116,22 @@ def test_all_24_bits_count(M, N, K):
     api.sgemm(x, w, out)
     err = [float((o.double() - ref).norm() / ref.norm()) for o in (api.gemm_f32_tc(x, w), out)]
     assert err[0] <= 3e-7 < err[1], err
+
+
+@pytest.mark.parametrize("M", [1, 3, 4, 5, 32])
+@pytest.mark.parametrize("N,K", [(300, 68), (40000, 260), (700, 2564)])
+def test_few_rows_give_the_bits_of_many(M, N, K):
+    """Tiles of at most 32 rows (two groups of converting warps; up to 4 rows taken apart by the product itself, from any address
+    that a float has) against tiles of 64: the same arithmetic, so the same bits. Tile heights that leave converting warps with
+    some rows, none or all; more units than blocks; a last chunk that is not whole; a gated product."""
+    x, w = rnd(M * K + 1, seed=11)[1:].view(M, K), rnd(N, K, seed=12)
+    nt = (M + 15) // 16 * 16
+    want = api.gemm_f32_tc(x, w, plan=(128, 64, False))
+    assert bool(((want.double() - x.double() @ w.double().T).abs() <= bound(x, w)).all())
+    for height in (128, 120, 65, 33, 32, 17):
+        assert torch.equal(api.gemm_f32_tc(x, w, plan=(height, nt, False)), want), height
+        assert torch.equal(api.gemm_f32_tc(x.clone(), w, plan=(height, nt, False)), want), height
+    gated = api.gemm_f32_tc(x, w, api.MODE_SILU, plan=(64, 64, False))
+    for height in (64, 60, 33, 24, 16):
+        assert torch.equal(api.gemm_f32_tc(x, w, api.MODE_SILU, plan=(height, nt, False)), gated), height
+    api.gemm_tc_check()
