@@ -446,8 +446,9 @@ def f32_plan(M, N, K, mode=MODE_STORE, allow_partial=False):
     takes the longest of its 24 mma (half a clock a row and 8, 150 a chunk between them), its conversion (1,150 measured where the
     mma are short: one row of 9,728 gated outputs takes 50 to 52 us with tiles of 28 to 16 outputs) and its bytes (of weights at a
     148th of the HBM rate, 24 a clock; of weights and pieces of x at 55 a clock from the L2); a unit 2,500 more to fill and drain.
-    Partial sums are read by their consumer at the same rate; adding a group into ``out`` costs a unit about 4,000 (544 rows, 2,560
-    outputs of 4,096: 97 us with groups added, 71 in parts). Sweeps of all plans at 1 to 1,000 rows of the 4B widths: what this
+    Partial sums are written and read by their consumer, together as long as 10 bytes each at the same rate (a norm of 544 rows takes
+    13.6 us behind seven parts, 5.1 behind one); adding a group into ``out`` costs a unit about 2,500 (its loads run beside the next
+    chunks' mma), into tensor memory 600. Sweeps of all plans at 1 to 1,000 rows of the 4B widths: what this
     picks is within 3 % of the best."""
     sms = sm_count()
     kb = (K + F32_CHUNK - 1) // F32_CHUNK
@@ -459,6 +460,8 @@ def f32_plan(M, N, K, mode=MODE_STORE, allow_partial=False):
     for row_tiles in range(fewest, fewest + 3):
         nt = ((M + row_tiles - 1) // row_tiles + 15) // 16 * 16
         row_tiles = (M + nt - 1) // nt
+        bufs = min(4, 512 // (nt + 96))
+        kept = bufs * (nt + 96) + nt <= 512            # room in tensor memory for the groups' sum
         for height in F32_TILE_HEIGHTS:
             tile_n = height // per_out
             bytes_w = per_out * tile_n * 256
@@ -466,8 +469,8 @@ def f32_plan(M, N, K, mode=MODE_STORE, allow_partial=False):
             tiles = (N + tile_n - 1) // tile_n
             for split in ((False, True) if allow_partial and groups > 1 and f32_rows_a_launch(M, K) == M else (False,)):
                 units = tiles * row_tiles * (groups if split else 1)
-                unit = (length if split else kb) * chunk + 2500 + (0 if split else (groups - 1) * 4000)
-                cost = -(-units // sms) * unit + (groups * M * N * 4 / (sms * 24) if split else 0)
+                unit = (length if split else kb) * chunk + 2500 + (0 if split else (groups - 1) * (600 if kept else 2500))
+                cost = -(-units // sms) * unit + (groups * M * N * 10 / (sms * 24) if split else 0)
                 if best is None or cost < best[0]:
                     best = cost, (tile_n, nt, split)
     return best[1]

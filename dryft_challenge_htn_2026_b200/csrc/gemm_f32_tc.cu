@@ -15,6 +15,8 @@
 //
 // Summation order: K in S groups of whole chunks, a group's chunks in order, then the groups in order. S depends on
 // (N, K) alone, and nothing else of the order on the number of rows: a row's result does not depend on the rows beside it.
+// A unit of several groups keeps their sum in tensor memory where there is room for it (544 rows, 2,560 outputs of 4,096: 97 us when
+// every group was added into the output); else it adds each into the output.
 // Where a unit of work holds one group (split) the groups leave as partial sums [S][M][N] for the consumer to add
 // up in the same order; where it holds all of them (few units otherwise) it adds group after group into ``out`` itself.
 //
@@ -34,7 +36,7 @@
 // Measured in a graph (2,560 wide layers of 9,728; one converting group, one mma warp, descriptors built at each mma and split_rows in
 // front of every product -> this kernel; sgemm before both): one row: q/k/v 16.4 -> 12.4 us, output projection 13.8 -> 9.6, gated
 // 60.9 -> 50.1, down 22.1 -> 18.0 (the weights' bytes take 9.6, 6.4, 30.5, 15.2), a head of 50,000 91 -> 82 (6.2 TB/s). 544 rows:
-// 118 -> 99, 112 -> 71, 354 -> 332, 166 -> 156.
+// 118 -> 86, 112 -> 63, 354 -> 330, 166 -> 150 (of which the sums kept in tensor memory 99 -> 86, 71 -> 63, 156 -> 150).
 // Infinities, NaN and numbers beyond bfloat16's largest: a piece times a zero piece is NaN where the product is not. A
 // thread that finds a sum that is not finite works that one out again by plain FMA from x and W.
 #include <cuda.h>
@@ -213,7 +215,8 @@ struct Product {
     float *out, *parts;          // parts: [S][M][N] where a unit holds one group
     int M, N, K, Kp;
     int tile_n, tiles, nt, row_tiles, groups, group_len, split;   // tile_n: outputs a tile (weight rows; mode 2: half of them)
-    int w_stages, x_stages, w_box, bufs;   // w_box: bytes between boxes of weights in shared memory; bufs: pieces of W, accumulators
+    int w_stages, x_stages, w_box, bufs, kept;   // w_box: bytes between boxes of weights in shared memory; bufs: pieces of W, accumulators
+    // kept: the sums of the groups so far stay in tensor memory, behind the buffers, until the last group
     float act_pos, act_neg;
 };
 
@@ -527,7 +530,30 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&acc_empty[b]);
                 }
-                // ---- the group's sums leave
+                // ---- the group's sums leave, or join those of the groups before it
+                const bool last = g1 == kb1;
+                if (MODE != 2 && p.kept) {
+                    const uint32_t sums = a_base + p.bufs * A_COLS + j0 + ((uint32_t)(q * 32) << 16);
+#pragma unroll
+                    for (int c = 0; c < HALF_COLS / 16; c++)
+                        if (c < pieces) {
+                            uint32_t v[16];
+                            if (g0 != kb0) {
+                                tmem_ld16(sums + c * 16, v);
+#pragma unroll
+                                for (int i = 0; i < 16; i++) tot[c * 16 + i] = __uint_as_float(v[i]) + tot[c * 16 + i];
+                            }
+                            if (!last) {
+#pragma unroll
+                                for (int i = 0; i < 16; i++) v[i] = __float_as_uint(tot[c * 16 + i]);
+                                tmem_st16(sums + c * 16, v);
+                            }
+                        }
+                    if (!last) {
+                        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                        continue;
+                    }
+                }
                 if (MODE == 2) {           // one group; gate sums in the warps of lanes 0..63, up sums in the others
 #pragma unroll
                     for (int c = 0; c < HALF_COLS; c += 32)
@@ -551,7 +577,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
                             asm volatile("bar.sync %0, 128;" ::"r"(1 + half) : "memory");
                         }
                 } else if (mine) {
-                    const bool first = g0 == kb0, last = g1 == kb1;
+                    const bool first = g0 == kb0 || p.kept;
                     const int rows = min(cols, p.M - m0 - j0);
                     float* dst = out + (size_t)(m0 + j0) * p.N + n;
 #pragma unroll
@@ -633,6 +659,7 @@ int launch_as(Product p, const bf16* pieces, int* err, cudaStream_t st) {
     p.w_box = (p.tile_n + 7) / 8 * 1024;                      // 128 bytes a row, boxes at multiples of the swizzle's 1024
     const int w_stage = (MODE == 2 ? 4 : 2) * p.w_box;
     p.bufs = 512 / (p.nt + A_COLS) < MAX_BUFS ? 512 / (p.nt + A_COLS) : MAX_BUFS;
+    p.kept = MODE != 2 && !p.split && p.groups > 1 && p.bufs * (p.nt + A_COLS) + p.nt <= 512;
     // a stage of x is free when its mma are done, a stage of W once it is converted (``bufs`` more wait in tensor memory)
     p.x_stages = p.nt > 64 ? 2 : 4;                           // even: see below
     p.w_stages = (int)((budget - (size_t)p.x_stages * x_stage) / w_stage);

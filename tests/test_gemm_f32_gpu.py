@@ -135,3 +135,24 @@ def test_few_rows_give_the_bits_of_many(M, N, K):
     for height in (64, 60, 33, 24, 16):
         assert torch.equal(api.gemm_f32_tc(x, w, api.MODE_SILU, plan=(height, nt, False)), gated), height
     api.gemm_tc_check()
+
+
+@pytest.mark.parametrize("nt", [16, 32, 48, 64, 96, 112])
+def test_groups_summed_in_tensor_memory_or_in_the_output(nt):
+    """A unit of several groups of K (the last one shorter): row tiles that leave tensor memory room for their sum (16, 48 to 96 rows)
+    and ones that do not, full and ragged, against the groups left in parts and added in order; xIELU on the finished sums only."""
+    M, N, K = 150, 200, 2884
+    groups, length = api.f32_groups(N, K)
+    assert groups > 2 and groups * length > (K + 63) // 64
+    x, w = rnd(M, K, seed=13), rnd(N, K, seed=14)
+    parts = api.gemm_f32_tc(x, w, plan=(128, 64, True)).ws
+    want = parts[0]
+    for p in parts[1:]:
+        want = want + p
+    assert bool(((want.double() - x.double() @ w.double().T).abs() <= bound(x, w)).all())
+    assert torch.equal(api.gemm_f32_tc(x, w, plan=(120, nt, False)), want)
+    x[3, 5] = float("inf")
+    out = api.gemm_f32_tc(x, w, plan=(128, nt, False))
+    keep = torch.arange(M, device=DEV) != 3
+    assert torch.equal(out[keep], want[keep]) and not bool(out[3].isfinite().any())
+    api.gemm_tc_check()
