@@ -278,7 +278,16 @@ def attention_generic(q, out, k_store, v_store, row_pos, row_seq, page_table, n_
 F32_ATTENTION_HEAD_DIMS = (64, 128)
 F32_ATTENTION_MAX_GROUP = 16        # query heads a kv head
 F32_DECODE_BYTES = 256 << 20        # most scratch memory for the pages' results of single tokens; more sequences go in several launches
-F32_TILE_ROWS = 64                  # rows (queries x the query heads of a kv head) a block of attention_prompt_f32 takes
+F32_TILE_ROWS, F32_SHORT_TILE_ROWS = 64, 32  # rows (queries x the query heads of a kv head) a block of attention_prompt_f32 takes
+
+
+def f32_tile_rows(n_tok, n_heads, n_kv_heads):
+    """Rows a tile for a step of ``n_tok`` rows: while all tiles of 64 are on the SMs at once (two each) the step takes as long as its
+    longest tile, and tiles of 32 take two thirds of that a page. Us in tiles of 64 and 32, 32 heads of 128: 100 tokens 29 and 19,
+    300 63 and 54, 544 (272 tiles) 125 and 112; 700 and 300 (504 tiles) 169 and 206, eight of 150 (640 tiles) 83 and 88."""
+    group = n_heads // n_kv_heads
+    tiles = -(-n_tok // (F32_TILE_ROWS // group)) * n_kv_heads
+    return F32_SHORT_TILE_ROWS if tiles <= 2 * sm_count() else F32_TILE_ROWS
 
 
 def _need_f32_attention(q, out, k_store, v_store, page_table, n_heads, n_kv_heads, head_dim):
@@ -289,15 +298,16 @@ def _need_f32_attention(q, out, k_store, v_store, page_table, n_heads, n_kv_head
         raise KernelError(f"float32 attention: head size {head_dim} (64 or 128) / heads {n_heads}:{n_kv_heads} not supported")
 
 
-def attention_prompt_f32(q, out, k_store, v_store, tiles, cu_q, seq_pos0, page_table, n_heads, n_kv_heads, head_dim, window, scale):
-    """Float32 attention of portions of prompts (head sizes 64 and 128). ``tiles`` lists tiles of F32_TILE_ROWS // (query heads a kv
-    head) queries as for ``attention_prefill_bf16``. A row gives the bits ``attention_decode_f32`` gives for it."""
+def attention_prompt_f32(q, out, k_store, v_store, tiles, cu_q, seq_pos0, page_table, n_heads, n_kv_heads, head_dim, window, scale,
+                         tile_rows=F32_TILE_ROWS):
+    """Float32 attention of portions of prompts (head sizes 64 and 128). ``tiles`` lists tiles of ``tile_rows`` (64 or 32) // (query
+    heads a kv head) queries as for ``attention_prefill_bf16``. A row gives the bits ``attention_decode_f32`` gives for it."""
     _need_f32_attention(q, out, k_store, v_store, page_table, n_heads, n_kv_heads, head_dim)
     _need(tiles, "tiles", torch.int32, 2), _need(cu_q, "cu_q", torch.int32, 1), _need(seq_pos0, "seq_pos0", torch.int32, 1)
     lib = _lib("attention_f32.cu", {"HD": head_dim})
-    _check(lib, lib.dk_attn_f32_prompt(_p(q), _p(out), _p(k_store), _p(v_store), _p(tiles), tiles.shape[0], _p(cu_q), _p(seq_pos0),
-                                       _p(page_table), page_table.shape[1], n_heads, n_kv_heads, int(window or 0), c_float(scale),
-                                       _stream()), "attention_prompt_f32")
+    _check(lib, lib.dk_attn_f32_prompt(_p(q), _p(out), _p(k_store), _p(v_store), _p(tiles), tiles.shape[0], int(tile_rows), _p(cu_q),
+                                       _p(seq_pos0), _p(page_table), page_table.shape[1], n_heads, n_kv_heads, int(window or 0),
+                                       c_float(scale), _stream()), "attention_prompt_f32")
 
 
 def attention_decode_f32(q, out, k_store, v_store, row_pos, page_table, n_heads, n_kv_heads, head_dim, window, scale):

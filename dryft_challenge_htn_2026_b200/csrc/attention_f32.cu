@@ -9,18 +9,20 @@
 // maximum, weights against that maximum, their sum (a fixed tree), P.V (one FMA chain over the page); then the page is merged
 // into what the pages before it gave (merge()).
 //
-//   prompts: a block takes 64 rows (64 / G queries of one sequence x the G query heads of one kv head) through its pages. Q, K, V
-//       in shared memory (K's place takes P afterwards: 98 KB, two blocks an SM); S = Q.K^T with 4 x 4 scores a thread, P.V with
-//       4 rows x HD / 16 columns a thread. Bound by the chain load - scores - weights - P.V of the longest tiles (9 pages at
-//       544 tokens, 17 us a page with two blocks an SM, of which the FMA pipe is busy 9). 544 tokens, 32 heads of 128: 920 us with a
-//       warp a row (a shuffle tree a key) -> 155 us.
+//   prompts: a block takes 64 or 32 rows (rows / G queries of one sequence x the G query heads of one kv head) through its pages. Q, K,
+//       V in shared memory (K's place takes P afterwards: 98 or 82 KB, two blocks an SM); S = Q.K^T with 4 x 4 (2 x 4) scores a
+//       thread, P.V with 4 (2) rows x HD / 16 columns a thread; keys that every row of the tile sees go four at a time, only the few
+//       behind them with a test a row. Bound by the chain load - scores - weights - P.V (9 us a page of 64 rows and SM with two
+//       blocks, of which the FMA pipe is busy 4.3; 5.8 a page of 32). The tiles with the most pages of all heads start first: with the
+//       tiles of one head after those of another the last head's longest tiles came last. 32 heads of 128: 100 tokens 33 -> 19 us,
+//       300 72 -> 54, 544 157 -> 112 (125 in tiles of 64), 1,000 394 -> 265, 4,000 3,970 -> 3,640.
 //   single tokens: a block a (sequence, kv head, page), the pages merged by a second kernel. 2 sequences of 100 tokens: 203 us with
 //       a warp a row, whose keys follow one another at 2 us each -> 7.2 + 2.3 us.
 #include "common.cuh"
 
 namespace {
 
-constexpr int ROWS = 64, THREADS = 256, LDK = HD + 4, LDP = DK_PAGE + 4, MAX_G = 16;
+constexpr int THREADS = 256, LDK = HD + 4, LDP = DK_PAGE + 4, MAX_G = 16;
 constexpr int CV = HD / 64;                               // float4 columns of P.V a thread
 
 // A page's (maximum mp, sum lp) into the running (m, l): the factors of the old and of the page's values.
@@ -88,14 +90,17 @@ __device__ __forceinline__ void weights(float (&s)[4], float scale, int key0, in
     for (int o = 8; o > 0; o >>= 1) lp = __fadd_rn(lp, __shfl_xor_sync(0xffffffffu, lp, o));
 }
 
+template <int ROWS>
 __global__ void __launch_bounds__(THREADS, 2)
 prompt_kernel(const float* q, float* out, const float* k_store, const float* v_store, const int* tiles, const int* cu_q,
               const int* seq_pos0, const int* page_table, int pt_stride, int nh, int nkv, int window, float scale) {
+    constexpr int NI = ROWS / 16;                           // rows a thread
     extern __shared__ __align__(16) float smem[];
     float *q_s = smem, *k_s = q_s + ROWS * HD, *p_s = k_s, *v_s = k_s + DK_PAGE * LDK;
     pdl_wait();
     pdl_launch_dependents();
-    const int seq = tiles[2 * blockIdx.x], q0 = tiles[2 * blockIdx.x + 1], kvh = blockIdx.y;
+    // kv heads run fastest: the tiles come with the most keys first, and those of all heads start first
+    const int tile = blockIdx.x / nkv, kvh = blockIdx.x - tile * nkv, seq = tiles[2 * tile], q0 = tiles[2 * tile + 1];
     const int G = nh / nkv, flat0 = cu_q[seq] + q0, rows = min(ROWS / G, cu_q[seq + 1] - flat0) * G;
     const int pos0 = seq_pos0[seq] + q0, last = pos0 + rows / G - 1;
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
@@ -104,12 +109,12 @@ prompt_kernel(const float* q, float* out, const float* k_store, const float* v_s
         const int r = i / (HD / 4), c = (i % (HD / 4)) * 4;
         if (r < rows) copy16(q_s + r * HD + c, q + ((size_t)(flat0 + r / G) * nh + kvh * G + r % G) * HD + c);
     }
-    const float* qr[4];
-    int pos[4], lo[4];
-    float m[4], l[4], acc[4][4 * CV];
+    const float* qr[NI];
+    int pos[NI], lo[NI];
+    float m[NI], l[NI], acc[NI][4 * CV];
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const int r = ty * 4 + i;
+    for (int i = 0; i < NI; i++) {
+        const int r = ty * NI + i;
         qr[i] = q_s + min(r, rows - 1) * HD;
         pos[i] = r < rows ? pos0 + r / G : -1;              // a row that is not there sees nothing
         lo[i] = window > 0 ? max(0, pos[i] - window + 1) : 0;
@@ -124,65 +129,64 @@ prompt_kernel(const float* q, float* out, const float* k_store, const float* v_s
         load_page(v_s, HD, v_store, page, nkv, kvh);
         copy_wait();
         __syncthreads();
-        float s[4][4] = {}, a[4], b[4];
-        scores<4>(s, qr, k_s, tx);
+        float s[NI][4] = {}, a[NI], b[NI];
+        scores<NI>(s, qr, k_s, tx);
         __syncthreads();                                    // P goes where K was
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
+        for (int i = 0; i < NI; i++) {
             float mp, lp;
             weights(s[i], scale, key0, lo[i], pos[i], tx, mp, lp);
             a[i] = 1.f, b[i] = -1.f;                       // negative: nothing of this page for the row
             if (mp != -INFINITY) merge(m[i], l[i], mp, lp, a[i], b[i]);
             else if (lp != 0.f) l[i] = lp;                  // a NaN among the scores and nothing finite
 #pragma unroll
-            for (int j = 0; j < 4; j++) p_s[(ty * 4 + i) * LDP + tx + 16 * j] = s[i][j];
+            for (int j = 0; j < 4; j++) p_s[(ty * NI + i) * LDP + tx + 16 * j] = s[i][j];
         }
         __syncthreads();
-        float o[4][4 * CV] = {};
-        const bool open = key0 + DK_PAGE - 1 <= pos0 && (window <= 0 || key0 >= last - window + 1);
-        if (open) {                                         // every row sees every key
+        float o[NI][4 * CV] = {};
+        // the page's first keys, as far as every row sees all of them (fours of them: none where a window cuts the page)
+        const int open = window <= 0 || key0 >= last - window + 1 ? min(DK_PAGE, max(0, pos0 - key0 + 1) & ~3) : 0;
 #pragma unroll 2
-            for (int j = 0; j < DK_PAGE; j += 4) {
-                float4 p[4];
+        for (int j = 0; j < open; j += 4) {
+            float4 p[NI];
 #pragma unroll
-                for (int i = 0; i < 4; i++) p[i] = *reinterpret_cast<const float4*>(p_s + (ty * 4 + i) * LDP + j);
+            for (int i = 0; i < NI; i++) p[i] = *reinterpret_cast<const float4*>(p_s + (ty * NI + i) * LDP + j);
 #pragma unroll
-                for (int e = 0; e < 4; e++)
+            for (int e = 0; e < 4; e++)
+#pragma unroll
+                for (int c = 0; c < CV; c++) {
+                    const float4 v = *reinterpret_cast<const float4*>(v_s + (j + e) * HD + c * 64 + tx * 4);
+#pragma unroll
+                    for (int i = 0; i < NI; i++) {
+                        const float w = e == 0 ? p[i].x : e == 1 ? p[i].y : e == 2 ? p[i].z : p[i].w;
+                        o[i][c * 4] = fmaf(w, v.x, o[i][c * 4]), o[i][c * 4 + 1] = fmaf(w, v.y, o[i][c * 4 + 1]);
+                        o[i][c * 4 + 2] = fmaf(w, v.z, o[i][c * 4 + 2]), o[i][c * 4 + 3] = fmaf(w, v.w, o[i][c * 4 + 3]);
+                    }
+                }
+        }
+        // a value that a row does not see must not meet its zero weight
+        for (int j = open; j < min(DK_PAGE, last - key0 + 1); j++)
+#pragma unroll
+            for (int i = 0; i < NI; i++)
+                if (key0 + j >= lo[i] && key0 + j <= pos[i]) {
+                    const float w = p_s[(ty * NI + i) * LDP + j];
 #pragma unroll
                     for (int c = 0; c < CV; c++) {
-                        const float4 v = *reinterpret_cast<const float4*>(v_s + (j + e) * HD + c * 64 + tx * 4);
-#pragma unroll
-                        for (int i = 0; i < 4; i++) {
-                            const float w = e == 0 ? p[i].x : e == 1 ? p[i].y : e == 2 ? p[i].z : p[i].w;
-                            o[i][c * 4] = fmaf(w, v.x, o[i][c * 4]), o[i][c * 4 + 1] = fmaf(w, v.y, o[i][c * 4 + 1]);
-                            o[i][c * 4 + 2] = fmaf(w, v.z, o[i][c * 4 + 2]), o[i][c * 4 + 3] = fmaf(w, v.w, o[i][c * 4 + 3]);
-                        }
+                        const float4 v = *reinterpret_cast<const float4*>(v_s + j * HD + c * 64 + tx * 4);
+                        o[i][c * 4] = fmaf(w, v.x, o[i][c * 4]), o[i][c * 4 + 1] = fmaf(w, v.y, o[i][c * 4 + 1]);
+                        o[i][c * 4 + 2] = fmaf(w, v.z, o[i][c * 4 + 2]), o[i][c * 4 + 3] = fmaf(w, v.w, o[i][c * 4 + 3]);
                     }
-            }
-        } else {                                            // a value that a row does not see must not meet its zero weight
-            for (int j = 0; j < DK_PAGE; j++)
+                }
 #pragma unroll
-                for (int i = 0; i < 4; i++)
-                    if (key0 + j >= lo[i] && key0 + j <= pos[i]) {
-                        const float w = p_s[(ty * 4 + i) * LDP + j];
-#pragma unroll
-                        for (int c = 0; c < CV; c++) {
-                            const float4 v = *reinterpret_cast<const float4*>(v_s + j * HD + c * 64 + tx * 4);
-                            o[i][c * 4] = fmaf(w, v.x, o[i][c * 4]), o[i][c * 4 + 1] = fmaf(w, v.y, o[i][c * 4 + 1]);
-                            o[i][c * 4 + 2] = fmaf(w, v.z, o[i][c * 4 + 2]), o[i][c * 4 + 3] = fmaf(w, v.w, o[i][c * 4 + 3]);
-                        }
-                    }
-        }
-#pragma unroll
-        for (int i = 0; i < 4; i++)
+        for (int i = 0; i < NI; i++)
             if (b[i] >= 0.f || b[i] != b[i])
 #pragma unroll
                 for (int c = 0; c < 4 * CV; c++) acc[i][c] = merged(acc[i][c], o[i][c], a[i], b[i]);
         __syncthreads();                                    // the next page goes over this one
     }
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const int r = ty * 4 + i;
+    for (int i = 0; i < NI; i++) {
+        const int r = ty * NI + i;
         if (r >= rows) continue;
         const float inv = 1.f / l[i];
         float* dst = out + ((size_t)(flat0 + r / G) * nh + kvh * G + r % G) * HD + tx * 4;
@@ -266,21 +270,33 @@ merge_kernel(const float* ws_acc, const float* ws_ml, float* out, const int* row
     out[head * HD + d] = pos >= 0 ? acc * (1.f / l) : 0.f;
 }
 
-}  // namespace
-
-// q, out [T][nh * HD]; k_store, v_store [pages][nkv][64][HD]; tiles [n][2] = (sequence, first query of a tile of 64 / (nh / nkv)
-// queries within its portion); cu_q [sequences + 1]; seq_pos0 [sequences]. Every row of q belongs to a sequence's portion.
-DK_EXPORT int dk_attn_f32_prompt(const float* q, float* out, const float* k_store, const float* v_store, const int* tiles, int n_tiles,
-                                 const int* cu_q, const int* seq_pos0, const int* page_table, int pt_stride, int nh, int nkv,
-                                 int window, float scale, cudaStream_t st) {
-    if (nkv < 1 || nh % nkv != 0 || nh / nkv > MAX_G || ((uintptr_t)q | (uintptr_t)out | (uintptr_t)k_store | (uintptr_t)v_store) % 16 != 0)
-        return (int)cudaErrorInvalidValue;
+template <int ROWS>
+int launch_prompt(const float* q, float* out, const float* k_store, const float* v_store, const int* tiles, int n_tiles, const int* cu_q,
+                  const int* seq_pos0, const int* page_table, int pt_stride, int nh, int nkv, int window, float scale, cudaStream_t st) {
+    if ((long long)n_tiles * nkv > 0x7fffffffLL) return (int)cudaErrorInvalidValue;
     constexpr size_t smem = (size_t)(ROWS * HD + DK_PAGE * LDK + DK_PAGE * HD) * sizeof(float);
     static_assert(ROWS * LDP <= DK_PAGE * LDK, "P takes K's place");
-    cudaError_t e = cudaFuncSetAttribute(prompt_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(prompt_kernel<ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
-    return dk_launch(prompt_kernel, dim3(n_tiles, nkv), dim3(THREADS), smem, st, q, out, k_store, v_store, tiles, cu_q, seq_pos0,
+    return dk_launch(prompt_kernel<ROWS>, dim3((unsigned)(n_tiles * nkv)), dim3(THREADS), smem, st, q, out, k_store, v_store, tiles, cu_q, seq_pos0,
                      page_table, pt_stride, nh, nkv, window, scale);
+}
+
+}  // namespace
+
+// q, out [T][nh * HD]; k_store, v_store [pages][nkv][64][HD]; tiles [n][2] = (sequence, first query of a tile of tile_rows / (nh / nkv)
+// queries within its portion), tile_rows 64 or 32; cu_q [sequences + 1]; seq_pos0 [sequences]. Every row of q belongs to a sequence's
+// portion.
+DK_EXPORT int dk_attn_f32_prompt(const float* q, float* out, const float* k_store, const float* v_store, const int* tiles, int n_tiles,
+                                 int tile_rows, const int* cu_q, const int* seq_pos0, const int* page_table, int pt_stride, int nh,
+                                 int nkv, int window, float scale, cudaStream_t st) {
+    if (nkv < 1 || nh % nkv != 0 || nh / nkv > MAX_G || ((uintptr_t)q | (uintptr_t)out | (uintptr_t)k_store | (uintptr_t)v_store) % 16 != 0)
+        return (int)cudaErrorInvalidValue;
+    if (tile_rows == 64)
+        return launch_prompt<64>(q, out, k_store, v_store, tiles, n_tiles, cu_q, seq_pos0, page_table, pt_stride, nh, nkv, window, scale, st);
+    if (tile_rows == 32)
+        return launch_prompt<32>(q, out, k_store, v_store, tiles, n_tiles, cu_q, seq_pos0, page_table, pt_stride, nh, nkv, window, scale, st);
+    return (int)cudaErrorInvalidValue;
 }
 
 // One token a sequence: q, out [n_seq][nh * HD], row_pos [n_seq] (negative: a padding row, zeros). ws_acc: n_seq * nh * pt_stride *

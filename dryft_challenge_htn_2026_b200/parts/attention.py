@@ -68,6 +68,7 @@ class GQAAttention(Part):
             and group <= api.F32_ATTENTION_MAX_GROUP
         self.tiles = QueryTiles(api.TC_TILE_ROWS if self.tc_prefill else api.MMA_TILE_ROWS) \
             if rt.dtype == torch.bfloat16 else QueryTiles(api.F32_TILE_ROWS // group) if self.paged_f32 else None
+        self.short_tiles = QueryTiles(api.F32_SHORT_TILE_ROWS // group) if self.paged_f32 else None    # for short steps (api.f32_tile_rows)
 
     def param_decls(self):
         s = self.spec
@@ -93,7 +94,7 @@ class GQAAttention(Part):
         return [self.w_qkv, self.w_o]
 
     def step_plans(self):
-        return [self.tiles] if self.tiles is not None else []
+        return [t for t in (self.tiles, self.short_tiles) if t is not None]
 
     def cache_requests(self):
         s = self.spec
@@ -153,8 +154,10 @@ class GQAAttention(Part):
         if self.paged_f32 and ctx.is_decode:
             api.attention_decode_f32(q, o, kv.k, kv.v, ctx.row_pos, table, nh, nkv, hd, window, s.scale)
         elif self.paged_f32:
-            api.attention_prompt_f32(q, o, kv.k, kv.v, ctx.plans[self.tiles.key], ctx.cu_q, ctx.seq_pos0, table, nh, nkv, hd, window,
-                                     s.scale)
+            rows = api.f32_tile_rows(ctx.n_tok, nh, nkv)
+            tiles = self.tiles if rows == api.F32_TILE_ROWS else self.short_tiles
+            api.attention_prompt_f32(q, o, kv.k, kv.v, ctx.plans[tiles.key], ctx.cu_q, ctx.seq_pos0, table, nh, nkv, hd, window,
+                                     s.scale, rows)
         elif dtype == torch.float32:
             api.attention_generic(q, o, kv.k, kv.v, ctx.row_pos, ctx.row_seq, table, nh, nkv, hd, window, s.scale)
         elif ctx.is_decode:

@@ -103,3 +103,22 @@ def test_refusals():
     q = rnd(3, 64, seed=8)
     with pytest.raises(api.KernelError):
         api.attention_decode_f32(q, torch.empty_like(q), s["k_store"], s["v_store"], s["row_pos"], s["table"], 2, 1, 32, 0, 0.1)
+
+
+@pytest.mark.parametrize("nh,nkv,hd,window", [(8, 2, 128, 0), (4, 4, 64, 0), (6, 2, 128, 90), (16, 1, 64, 7), (10, 2, 64, 64), (3, 1, 128, 0)])
+def test_short_tiles_give_the_bits_of_long_ones(nh, nkv, hd, window):
+    """Tiles of 32 rows against tiles of 64 (5 and 3 heads a kv head leave rows of both unused): the same order of arithmetic a row;
+    portions that start and end anywhere in a page, and what no token wrote is NaN."""
+    before, new = [0, 100, 0, 63, 130, 640, 3], [70, 150, 1, 2, 65, 17, 62]
+    s = paged_setup(before, new, nkv, hd, torch.float32, seed=15)
+    s["k_store"].masked_fill_(s["k_store"] == 0, float("nan"))
+    s["v_store"].masked_fill_(s["v_store"] == 0, float("nan"))
+    q, out = rnd(s["n_tok"], nh * hd, seed=16), []
+    for rows in (api.F32_TILE_ROWS, api.F32_SHORT_TILE_ROWS):
+        plan = torch.tensor(QueryTiles(rows // (nh // nkv)).build(new, before, False), device=DEV)
+        out.append(torch.full_like(q, float("nan")))
+        api.attention_prompt_f32(q, out[-1], s["k_store"], s["v_store"], plan, s["cu_q"], s["pos0"], s["table"], nh, nkv, hd, window,
+                                 hd ** -0.5, rows)
+    assert torch.equal(out[0], out[1]) and bool(out[0].isfinite().all())
+    with pytest.raises(api.KernelError):
+        api.attention_prompt_f32(q, out[0], s["k_store"], s["v_store"], plan, s["cu_q"], s["pos0"], s["table"], nh, nkv, hd, window, 0.1, 48)
