@@ -73,3 +73,51 @@ def test_norm_rotation_and_cache_write_of_float32_rows(dtype, hd, nh, nkv, rows,
                                    1e-6, dense_out=dense)
             near(dense[live].view(-1, heads, hd), want(norm, False), dtype, parts + hd)
             assert bool((dense[pos < 0] == 7.0).all())
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("H,shift", [(4, 0), (516, 0), (2560, 0), (8192, 0), (2560, 1), (8196, 0), (258, 0)])
+def test_embedding_with_a_position_vector(dtype, H, shift):
+    """Rows of whole fours up to 8,192 on 16-byte boundaries, and rows that are not; a padding row, token ids out of range, far positions."""
+    V, rows = 40, 5
+    embed = rnd(V * H + shift, seed=5).to(dtype)[shift:].view(V, H)
+    tok = torch.tensor([3, 39, 0, 99, -2], dtype=torch.int32, device=DEV)
+    pos = torch.tensor([0, 1, -1, 100000, 777], dtype=torch.int32, device=DEV)
+    inv = 10000.0 ** (-torch.arange(0, H, 2, device=DEV, dtype=torch.float64) / H)
+    w = 1 + 0.1 * rnd(H, seed=6)
+    for table, weight in ((inv, w), (None, w), (inv, None)):
+        h, a = torch.full((rows, H), 7.0, device=DEV), torch.full((rows, H), 7.0, dtype=dtype, device=DEV)
+        api.embed_position_rmsnorm(tok, embed, 1.5, pos, table, weight, 1e-6, h, a)
+        want = embed[tok.long().clamp(0, V - 1)].double() * 1.5
+        if table is not None:
+            ang = pos.clamp(min=0).double()[:, None] * inv
+            want = want + torch.stack([ang.sin(), ang.cos()], -1).view(rows, -1)
+        near(h, want, torch.float32)
+        if weight is not None:
+            near(a, want * torch.rsqrt(want.pow(2).mean(-1, keepdim=True) + 1e-6) * w.double(), dtype, H)
+        else:
+            assert bool((a == 7.0).all())
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("nkv,hd,hdv,extra,shift", [(8, 128, 128, 0, 0), (2, 64, 32, 8, 0), (3, 20, 12, 0, 0), (1, 128, 128, 3, 0),
+                                                   (2, 64, 64, 0, 1), (1, 576, 0, 0, 0)])
+def test_keys_and_values_into_the_cache(dtype, nkv, hd, hdv, extra, shift):
+    """Rows of wider matrices, heads and rows of whole 16-byte pieces and not, addresses off them, padding rows, and no values of their own to store."""
+    rows, ld = 7, nkv * (hd + hdv) + extra
+    proj = rnd(rows * ld + shift, seed=7).to(dtype)[shift:].view(rows, ld)
+    k, v = proj[:, :nkv * hd], proj[:, nkv * hd:nkv * (hd + hdv)] if hdv else proj[:, :nkv * hd]
+    ks = torch.full((4, nkv, 64, hd), 7.0, dtype=dtype, device=DEV)
+    vs = torch.full((4, nkv, 64, hdv), 7.0, dtype=dtype, device=DEV) if hdv else None
+    pos = torch.tensor([0, 63, 64, 100, -1, 5, 127], dtype=torch.int32, device=DEV)
+    seq = torch.tensor([0, 0, 0, 0, 1, 1, 1], dtype=torch.int32, device=DEV)
+    table = torch.tensor([[2, 0], [3, 1]], dtype=torch.int32, device=DEV)
+    api.kv_write(k, v, ks, vs, pos, seq, table, nkv, hd, hdv if hdv else hd)
+    live = (pos >= 0).nonzero().flatten()
+    pages, slots = table[seq[live].long(), (pos[live] // 64).long()].long(), (pos[live] % 64).long()
+    for store, x, d in ((ks, k, hd), (vs, v, hdv)):
+        if store is None:
+            continue
+        want = torch.full_like(store, 7.0)
+        want[pages, :, slots] = x[live].reshape(len(live), nkv, d)
+        assert torch.equal(store, want)
