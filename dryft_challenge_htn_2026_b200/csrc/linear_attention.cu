@@ -40,26 +40,33 @@ linear_attention_step_kernel(const T* q, const T* k, const T* v, long long ld, f
     float* sv = sk + LA_TB * hd;                 // [LA_TB][cslice]
     float* part = sv + LA_TB * cslice;           // [LA_TB][R][cols_pad]
     float* sd = part + LA_TB * LA_THREADS;       // [LA_TB][hd], GATED only
-    pdl_wait();
-    pdl_launch_dependents();
+    // Single tokens: positions, slots, decays and the state itself, which no other kernel of a step writes, are requested before the
+    // wait for the kernel that makes q, k and v. (Portions are launched whole.)
+    const bool early = cu_q == nullptr;
+    if (!early) pdl_wait();
     const int s = blockIdx.x, h = blockIdx.y, col0 = blockIdx.z * cslice;
     const int cols = min(cslice, hdv - col0);            // value columns of this block: [col0, col0 + cols)
     const int r0 = cu_q ? cu_q[s] : s, r1 = cu_q ? cu_q[s + 1] : s + 1;
     const int tid = threadIdx.x, c = tid % cols_pad, rg = tid / cols_pad;
     const size_t ow = (size_t)nh * hdv;
-    if (seq_pos0[s] < 0) {
+    const int pos0 = seq_pos0[s], slot = seq_slot[s];
+    const float d = GATED ? 0.f : decay[h];
+    if (pos0 < 0) {
+        if (early) pdl_wait();
+        pdl_launch_dependents();
         for (int t = r0; t < r1; t++)
             for (int i = tid; i < cols; i += LA_THREADS) out[(size_t)t * ow + (size_t)h * hdv + col0 + i] = 0.f;
         return;
     }
-    const float d = GATED ? 0.f : decay[h];
-    float* S = state + ((size_t)seq_slot[s] * nh + h) * (size_t)hd * hdv + col0;
+    float* S = state + ((size_t)slot * nh + h) * (size_t)hd * hdv + col0;
     float st[EPT];
 #pragma unroll
     for (int i = 0; i < EPT; i++) {
         const int row = rg + R * i;
         st[i] = (row < hd && c < cols) ? S[(size_t)row * hdv + c] : 0.f;
     }
+    if (early) pdl_wait();
+    pdl_launch_dependents();
     for (int t0 = r0; t0 < r1; t0 += LA_TB) {
         const int nt = min(LA_TB, r1 - t0);
         __syncthreads();
