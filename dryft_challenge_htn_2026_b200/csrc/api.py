@@ -460,8 +460,8 @@ def f32_plan(M, N, K, mode=MODE_STORE, allow_partial=False):
     148th of the HBM rate, 24 a clock; of weights and pieces of x at 55 a clock from the L2); a unit 2,500 more to fill and drain.
     Partial sums are written and read by their consumer, together as long as 10 bytes each at the same rate (a norm of 544 rows takes
     13.6 us behind seven parts, 5.1 behind one); adding a group into ``out`` costs a unit about 2,500 (its loads run beside the next
-    chunks' mma), into tensor memory 600. Sweeps of all plans at 1 to 1,000 rows of the 4B widths: what this
-    picks is within 3 % of the best."""
+    chunks' mma), into tensor memory 600. Sweeps of all plans of the 4B widths: what this picks is within
+    3 % of the best up to 32 rows and mostly 5 % beyond (q/k/v at 161 rows 38 us against 34, at 1,000 158 against 144)."""
     sms = sm_count()
     kb = (K + F32_CHUNK - 1) // F32_CHUNK
     groups, length = f32_groups(N, K, mode)
@@ -775,10 +775,11 @@ def skinny_tc_plan(M, N, K, mode, allow_partial=False):
             tiles = (N + bn // 2 - 1) // (bn // 2)
             return bn * -(-tiles // sms)
         return min(TC_TILE_HEIGHTS, key=lambda bn: (span(bn), bn)), 1
-    if mode == MODE_XIELU:        # no slices (the activation needs whole sums): the tile height with the smallest unit
-        return min(TC_TILE_HEIGHTS, key=lambda bn: (bn * -(-((N + bn - 1) // bn) // sms), bn)), 1
     if mode != MODE_STORE or not allow_partial:
-        return 256, 1
+        # no slices (an activation needs whole sums, a caller a tensor): the tile height that gives an SM the fewest rows to stream.
+        # A head of 151,936 of 2,560 in tiles of 256 rows (594, two more than four a block): 121 us at 9 rows, 124 at 16, 133 at 64; of
+        # 208 (731, under five) 113, 112, 126; one of 32,768 at 16 rows 28.3 (256), 27.4 (224); 2,560 of 4,096 at 64 23.9 (256), 21.2 (128).
+        return min(TC_TILE_HEIGHTS, key=lambda bn: (bn * -(-((N + bn - 1) // bn) // sms), bn)), 1
     if M <= 32:
         plan = _few_units_plan(N, kb, sms)
         if plan is not None:

@@ -49,6 +49,16 @@ def test_skinny_tc_plan_gives_every_slice_work_and_no_more_units_than_sms():
         assert api.skinny_tc_plan(64, 4096, 4096, api.MODE_STORE, True) == (144, 5)
 
 
+def test_a_product_without_slices_gives_an_sm_the_fewest_rows_to_stream():
+    for mode in (api.MODE_STORE, api.MODE_STORE_F32, api.MODE_XIELU):
+        for M, N in itertools.product((9, 128), (40, 2560, 32768, 151936)):
+            bn, sk = api.skinny_tc_plan(M, N, 2560, mode)
+            rows = [b * -(-(-(-N // b)) // api.sm_count()) for b in (bn,) + api.TC_TILE_HEIGHTS]
+            assert sk == 1 and rows[0] == min(rows)
+    if api.sm_count() == 148:
+        assert api.skinny_tc_plan(16, 151936, 2560, api.MODE_STORE_F32) == (208, 1)
+
+
 def test_decode_splits_depend_on_the_batch_only_and_stay_within_what_the_merge_takes():
     seen = {}
     for n_seq, nkv, group in itertools.product((1, 2, 8, 16, 32, 64, 128, 500), (1, 2, 8), (1, 4, 16, 20)):

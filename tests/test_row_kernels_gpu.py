@@ -121,3 +121,42 @@ def test_keys_and_values_into_the_cache(dtype, nkv, hd, hdv, extra, shift):
         want = torch.full_like(store, 7.0)
         want[pages, :, slots] = x[live].reshape(len(live), nkv, d)
         assert torch.equal(store, want)
+
+
+@pytest.mark.parametrize("M,N", [(9, 40000), (128, 31000), (33, 2564)])
+def test_heads_of_every_tile_height(M, N):
+    """The decode form of the tensor-core product with a float32 result, several tiles a block, a last one that is not full."""
+    K = 136
+    x, w = rnd(M, K, seed=8).to(torch.bfloat16), rnd(N, K, seed=9, scale=K ** -0.5).to(torch.bfloat16)
+    want = x.double() @ w.double().t()
+    for bn in api.TC_TILE_HEIGHTS:
+        out = torch.full((M, N), float("nan"), device=DEV)
+        api.gemm_tc(x, w, api.MODE_STORE_F32, out, (bn, 1))
+        assert bool(((out.double() - want).abs() <= K * 2.0 ** -23 * (x.double().abs() @ w.double().abs().t())).all()), bn
+    api.gemm_tc_check()
+
+
+@pytest.mark.parametrize("lens", [[130] * 8, [64, 1, 200, 63, 65, 300, 2, 128], [70] * 4])
+def test_recurrence_in_chunks_of_64_value_columns(lens):
+    """Heads enough for blocks of 64 value columns (and, in four sequences of 16 heads, for blocks of 32) against the plain recurrence
+    in float64: outputs and states; silu of q, k and v is rounded to bfloat16 as the kernel rounds it."""
+    nh, hd, T, n = 16, 128, sum(lens), len(lens)
+    proj = rnd(T, 3 * nh * hd, seed=10).to(torch.bfloat16)
+    decay = 1.0 - 2.0 ** -(2 + 4 * torch.arange(nh, device=DEV, dtype=torch.float32) / nh)
+    state = rnd(n, nh, hd, hd, seed=11)
+    cu = torch.tensor([0] + torch.tensor(lens).cumsum(0).tolist(), dtype=torch.int32, device=DEV)
+    act = torch.nn.functional.silu(proj.float()).to(torch.bfloat16).double().view(T, 3, nh, hd)
+    want, last = torch.empty(T, nh, hd, dtype=torch.float64, device=DEV), state.double()
+    for s in range(n):
+        S = last[s]
+        for t in range(int(cu[s]), int(cu[s + 1])):
+            S = decay.double()[:, None, None] * S + act[t, 1][:, :, None] * act[t, 2][:, None, :]
+            want[t] = (act[t, 0][:, :, None] * S).sum(1)
+        last[s] = S
+    out = torch.full((T, nh * hd), float("nan"), device=DEV)
+    slot = torch.arange(n, dtype=torch.int32, device=DEV)
+    q, k, v = proj.split(nh * hd, 1)
+    api.linear_attention_chunk_bf16(q, k, v, out, state, cu, slot, decay, n, nh, hd, hd)
+    # scores and weights are bfloat16 operands of the products: 2^-8 of the terms' norm, states 2^-16
+    assert float((out.double().view_as(want) - want).norm() / want.norm()) <= 2.0 ** -7
+    assert float((state.double() - last).norm() / last.norm()) <= 2.0 ** -13
