@@ -159,6 +159,9 @@ __global__ void silu_mul_kernel(const T* gu, T* out, size_t n, int I) {
 }
 
 // ---------------------------------------------------------------------------------------------
+// A head's sum of squares is that of its pairs' (d, d + hd/2): a lane's pairs in order, then the lanes by halves (warp_sum).
+__device__ __forceinline__ float pair_squares(float first, float second) { return fmaf(first, first, __fmul_rn(second, second)); }
+
 // One warp per (token, head) over nh query heads, nkv key heads and nkv value heads of a fused
 // projection row qkv[t] = [q | k | v]. Query and key heads: optional RMSNorm over the head
 // (weights qn / kn), optional rotate-half rotation by the angle table at the token's position.
@@ -247,7 +250,7 @@ __global__ void qk_norm_rope_write_kernel(const T* qkv, const float* parts, int 
     if (nw) {
         float ss = 0.f;
 #pragma unroll
-        for (int i = 0; i < 4; i++) ss += x1[i] * x1[i] + x2[i] * x2[i];
+        for (int i = 0; i < 4; i++) ss += pair_squares(x1[i], x2[i]);
         ss = warp_sum(ss);
         const float rs = rsqrtf(ss / (float)hd + eps);
 #pragma unroll
@@ -268,12 +271,39 @@ __global__ void qk_norm_rope_write_kernel(const T* qkv, const float* parts, int 
     }
 }
 
+// The head's sum of squares in the order of qk_norm_rope_write_kernel, whose lane L holds the pairs L and (heads of 128) L + 32: here
+// pairs 4 l + c lie with lane l of each half of the head, c = 0..3. The 8 lanes of a quarter of the head (heads of 64: of a half) add
+// up one c (two); 10 shuffles with the caller's four instead of 24.
+template <int HDT>
+__device__ __forceinline__ float head_squares(const float4& first, const float4& other, int lane) {
+    const float t[4] = {pair_squares(first.x, other.x), pair_squares(first.y, other.y), pair_squares(first.z, other.z),
+                        pair_squares(first.w, other.w)};
+    const bool odd = (lane & 8) != 0, high = (lane & 16) != 0;
+    float s;
+    if constexpr (HDT == 128) {                               // quarters 0 and 2 hold pairs 0..31 and c = 0, 2; 1 and 3 32..63 and c = 1, 3
+        const float a = high ? t[2] : t[0], b = high ? t[3] : t[1];
+        s = odd ? b : a;
+        s += __shfl_xor_sync(0xffffffffu, odd ? a : b, 8);    // pair L + 32 to pair L
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        s += __shfl_xor_sync(0xffffffffu, s, 16);             // c with c ^ 2
+    } else {                                                  // halves 0 and 1: c = 0, 2 and c = 1, 3
+        float u = odd ? t[3] : t[2];
+        s = odd ? t[1] : t[0];
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o), u += __shfl_xor_sync(0xffffffffu, u, o);
+        s += u;
+    }
+    return s + __shfl_xor_sync(0xffffffffu, s, 8);            // c with c ^ 1
+}
+
 // The same for heads of 64 or 128 whose rows are float32 (parts of a projection, or a float32 projection as its only part): a lane has 4
 // consecutive columns of a head and reads them as one float4 of every part, up to eight parts on their way at a time; the other half
-// of the rotation comes from the lane half a head further. Bound by the trip to the L2 after the wait. In a chain of its own, with
+// of the rotation comes from the lane half a head further. Every sum, the squares' among them, is added up as above, so that a row's
+// result does not depend on where its tensors lie. Bound by the trip to the L2 after the wait. In a chain of its own, with
 // scalar loads before: 4 parts of one row of 48 heads of 128 3.6 -> 1.8 us, 9 parts of 64 rows 6.0 -> 3.1, 544 float32 rows 12.2 -> 10.9.
 template <typename T, int HDT>
-__global__ void qk_norm_rope_write_quad_kernel(const float* parts, int n_parts, size_t part_stride, T* q_out, T* dense_out,
+__global__ void qk_norm_rope_write_quad_kernel(const float* parts, int n_parts, size_t part_stride, float zero, T* q_out, T* dense_out,
                                                const float* __restrict__ qn, const float* __restrict__ kn,
                                                const float* __restrict__ cos_t, const float* __restrict__ sin_t, const int* row_pos,
                                                const int* row_seq, const int* page_table, int pt_stride, T* k_store, T* v_store,
@@ -288,7 +318,7 @@ __global__ void qk_norm_rope_write_quad_kernel(const float* parts, int n_parts, 
     const bool is_q = hidx < nh, is_v = hidx >= nh + nkv;
     const bool work = pos >= 0 && (is_q || write_kv || dense_out != nullptr);
     T* dst = nullptr;
-    float4 c = make_float4(1.f, 1.f, 1.f, 1.f), sn = make_float4(0.f, 0.f, 0.f, 0.f), w = c;
+    float4 c = make_float4(1.f, 1.f, 1.f, 1.f), sn = make_float4(0.f, 0.f, 0.f, 0.f), w = c, wy = c;
     const float* nw = is_v ? nullptr : is_q ? qn : kn;
     const bool turn = cos_t != nullptr && !is_v;
     if (work) {
@@ -304,11 +334,11 @@ __global__ void qk_norm_rope_write_quad_kernel(const float* parts, int n_parts, 
             c = *reinterpret_cast<const float4*>(cos_t + (size_t)pos * HALF + d % HALF);
             sn = *reinterpret_cast<const float4*>(sin_t + (size_t)pos * HALF + d % HALF);
         }
-        if (nw) w = *reinterpret_cast<const float4*>(nw + d);
+        if (nw) w = *reinterpret_cast<const float4*>(nw + d), wy = *reinterpret_cast<const float4*>(nw + (d ^ HALF));
     }
     pdl_launch_dependents();   // before the wait, as in qk_norm_rope_write_kernel
     pdl_wait();
-    float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 x = make_float4(zero, zero, zero, zero);
     if (work) {
         const float* p = parts + (size_t)t * heads * HDT + (size_t)hidx * HDT + d;
         for (int k = 0; k < n_parts; k += 8) {
@@ -321,19 +351,19 @@ __global__ void qk_norm_rope_write_quad_kernel(const float* parts, int n_parts, 
                 if (k + u < n_parts) x.x += v[u].x, x.y += v[u].y, x.z += v[u].z, x.w += v[u].w;
         }
     }
-    float ss = (x.x * x.x + x.y * x.y) + (x.z * x.z + x.w * x.w);
-#pragma unroll
-    for (int o = G / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-    if (nw) {
-        const float rs = rsqrtf(ss / (float)HDT + eps);
-        x.x = x.x * rs * w.x, x.y = x.y * rs * w.y, x.z = x.z * rs * w.z, x.w = x.w * rs * w.w;
-    }
     float4 y;                                                 // the same columns of the head's other half
     y.x = __shfl_xor_sync(0xffffffffu, x.x, G / 2), y.y = __shfl_xor_sync(0xffffffffu, x.y, G / 2);
     y.z = __shfl_xor_sync(0xffffffffu, x.z, G / 2), y.w = __shfl_xor_sync(0xffffffffu, x.w, G / 2);
+    const bool second = d >= HALF;
+    const float ss = head_squares<HDT>(second ? y : x, second ? x : y, lane);
+    if (nw) {
+        const float rs = rsqrtf(ss / (float)HDT + eps);
+        x.x = x.x * rs * w.x, x.y = x.y * rs * w.y, x.z = x.z * rs * w.z, x.w = x.w * rs * w.w;
+        y.x = y.x * rs * wy.x, y.y = y.y * rs * wy.y, y.z = y.z * rs * wy.z, y.w = y.w * rs * wy.w;
+    }
     if (!work) return;
     if (turn) {
-        if (d < HALF)
+        if (!second)
             x = make_float4(x.x * c.x - y.x * sn.x, x.y * c.y - y.y * sn.y, x.z * c.z - y.z * sn.z, x.w * c.w - y.w * sn.w);
         else
             x = make_float4(x.x * c.x + y.x * sn.x, x.y * c.y + y.y * sn.y, x.z * c.z + y.z * sn.z, x.w * c.w + y.w * sn.w);
@@ -662,7 +692,7 @@ DK_EXPORT int dk_qk_norm_rope_write(int dtype, const void* qkv, const float* par
         const int n = parts != nullptr ? n_parts : 1;
 #define ROPE_QUAD(HDT)                                                                                                   \
     DISPATCH_T(dtype, return dk_launch(qk_norm_rope_write_quad_kernel<T, HDT>, dim3((unsigned)((warps * HDT + 511) / 512)), dim3(128), 0, st, \
-                                       rows32, n, (size_t)part_stride, (T*)q_out, (T*)dense_out, qn, kn, cos_t, sin_t, row_pos,        \
+                                       rows32, n, (size_t)part_stride, parts != nullptr ? 0.f : -0.f, (T*)q_out, (T*)dense_out, qn, kn, cos_t, sin_t, row_pos,        \
                                        row_seq, page_table, pt_stride, (T*)k_store, (T*)v_store, n_tok, nh, nkv, eps, write_kv))
         if (hd == 128) ROPE_QUAD(128);
         ROPE_QUAD(64);

@@ -76,6 +76,35 @@ def test_norm_rotation_and_cache_write_of_float32_rows(dtype, hd, nh, nkv, rows,
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("hd,nh,nkv", [(64, 3, 1), (128, 4, 2)])
+@pytest.mark.parametrize("rows,parts", [(1, 1), (33, 4), (70, 9)])
+def test_norm_and_rotation_give_the_same_bits_wherever_the_rows_lie(dtype, hd, nh, nkv, rows, parts):
+    """Rows on 16-byte boundaries (four columns a lane) and 4 bytes off them (a number at a time): one order of every sum. In float32
+    numbers of any exponent and zeros of both signs beside them, whose last bit shows a different order."""
+    heads = nh + 2 * nkv
+    ws = rnd(parts * rows * heads * hd, seed=12) * torch.exp2(torch.randint(-9, 9, (parts * rows * heads * hd,), device=DEV))
+    ws[::17] = -0.0
+    qn, kn, ang = 1 + 0.1 * rnd(hd, seed=13), 1 + 0.1 * rnd(hd, seed=14), rnd(200, hd // 2, seed=15)
+    pos = (torch.arange(rows, dtype=torch.int32, device=DEV) * 37) % 190
+    seq = torch.arange(rows, dtype=torch.int32, device=DEV)
+    table = torch.arange(rows * 3, dtype=torch.int32, device=DEV).view(rows, 3)
+    for direct in (False, True) if dtype == torch.float32 and parts == 1 else (False,):
+        got = []
+        for off in (0, 1):
+            flat = torch.empty(ws.numel() + 4, device=DEV)[off:off + ws.numel()]
+            src = flat.copy_(ws).view(parts, rows, heads * hd)
+            q = torch.zeros(rows, nh * hd, dtype=dtype, device=DEV)
+            k = torch.zeros(rows * 3, nkv, 64, hd, dtype=dtype, device=DEV)
+            v = k.clone()
+            api.qk_norm_rope_write(src[0] if direct else api.Partial(src), q, qn, kn, ang.cos(), ang.sin(), pos, seq, table, k, v, nh, nkv,
+                                   hd, 1e-6)
+            bits = torch.int16 if dtype == torch.bfloat16 else torch.int32
+            got.append([t.view(bits) for t in (q, k, v)])
+        for a, b in zip(*got):
+            assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("H,shift", [(4, 0), (516, 0), (2560, 0), (8192, 0), (2560, 1), (8196, 0), (258, 0)])
 def test_embedding_with_a_position_vector(dtype, H, shift):
     """Rows of whole fours up to 8,192 on 16-byte boundaries, and rows that are not; a padding row, token ids out of range, far positions."""
