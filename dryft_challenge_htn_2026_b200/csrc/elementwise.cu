@@ -729,14 +729,14 @@ __global__ void embed_position_rmsnorm_kernel(const int* tok, const T* __restric
     float* hr = h + row * H;
     float ss = 0.f;
     for (int i = threadIdx.x; i < H; i += blockDim.x) {
-        float v = to_f(e[i]) * scale;
+        float v = __fmul_rn(to_f(e[i]), scale);
         if (inv_freq && (i >> 1) < H / 2) {
             double ang = (double)p * inv_freq[i >> 1];
             ang -= 6.283185307179586476925 * rint(ang * 0.15915494309189533577);
-            v += (i & 1) ? cosf((float)ang) : sinf((float)ang);
+            v = __fadd_rn(v, (i & 1) ? cosf((float)ang) : sinf((float)ang));
         }
         hr[i] = v;
-        ss += v * v;
+        ss = fmaf(v, v, ss);
     }
     ss = block_sum(ss, red);
     if (w == nullptr) return;
@@ -746,14 +746,16 @@ __global__ void embed_position_rmsnorm_kernel(const int* tok, const T* __restric
 }
 
 // The same for widths that are multiples of 4, up to 8,192, on 16-byte boundaries: a thread holds up to four fours of columns, and an
-// angle's sine and cosine are worked out together, once. Bound by the sines and the
-// float64 angles. (16,000 rows of 2,560, bfloat16: 195 us with every number's angle worked out by itself, now 119.)
+// angle's sine and cosine are worked out together, once. The bits are those of the kernel above: product and sine are rounded apart,
+// and the squares, handed over in shared memory, are added up in its order (a row's start does not depend on where its tensors lie).
+// Bound by the sines and the float64 angles. (16,000 rows of 2,560, bfloat16: 195 us with every number's angle worked out by itself, now 119.)
 template <typename T>
 __global__ void __launch_bounds__(512)
 embed_position_rmsnorm_wide_kernel(const int* tok, const T* __restrict__ embed, float scale, const int* row_pos,
                                    const double* __restrict__ inv_freq, const float* __restrict__ w, float eps, int H, int V, float* h,
                                    T* a) {
     __shared__ float red[33];
+    extern __shared__ __align__(16) float vrow[];        // [H]
     pdl_launch_dependents();
     pdl_wait();
     const size_t row = blockIdx.x;
@@ -761,7 +763,7 @@ embed_position_rmsnorm_wide_kernel(const int* tok, const T* __restrict__ embed, 
     t = t < 0 ? 0 : (t >= V ? V - 1 : t);
     const int p = inv_freq ? max(row_pos[row], 0) : 0;
     const T* e = embed + (size_t)t * H;
-    float v[4][4], ss = 0.f;
+    float v[4][4];
 #pragma unroll
     for (int k = 0; k < 4; k++) {
         const int i = (k * blockDim.x + threadIdx.x) * 4;
@@ -771,20 +773,25 @@ embed_position_rmsnorm_wide_kernel(const int* tok, const T* __restrict__ embed, 
         else *reinterpret_cast<uint2*>(x) = *reinterpret_cast<const uint2*>(e + i);
 #pragma unroll
         for (int c = 0; c < 4; c += 2) {
-            v[k][c] = to_f(x[c]) * scale, v[k][c + 1] = to_f(x[c + 1]) * scale;
+            v[k][c] = __fmul_rn(to_f(x[c]), scale), v[k][c + 1] = __fmul_rn(to_f(x[c + 1]), scale);
             if (inv_freq) {
                 double ang = (double)p * inv_freq[(i + c) >> 1];
                 ang -= 6.283185307179586476925 * rint(ang * 0.15915494309189533577);
                 float s, co;
                 sincosf((float)ang, &s, &co);
-                v[k][c] += s, v[k][c + 1] += co;
+                v[k][c] = __fadd_rn(v[k][c], s), v[k][c + 1] = __fadd_rn(v[k][c + 1], co);
             }
-            ss += v[k][c] * v[k][c] + v[k][c + 1] * v[k][c + 1];
         }
-        *reinterpret_cast<float4*>(h + row * H + i) = make_float4(v[k][0], v[k][1], v[k][2], v[k][3]);
+        const float4 f = make_float4(v[k][0], v[k][1], v[k][2], v[k][3]);
+        *reinterpret_cast<float4*>(h + row * H + i) = f;
+        *reinterpret_cast<float4*>(vrow + i) = f;
     }
-    ss = block_sum(ss, red);
     if (w == nullptr) return;
+    __syncthreads();
+    float ss = 0.f;
+#pragma unroll 4
+    for (int i = threadIdx.x; i < H; i += blockDim.x) ss = fmaf(vrow[i], vrow[i], ss);
+    ss = block_sum(ss, red);
     const float rs = rsqrtf(ss / (float)H + eps);
 #pragma unroll
     for (int k = 0; k < 4; k++) {
@@ -801,9 +808,9 @@ DK_EXPORT int dk_embed_position_rmsnorm(int dtype, const int* tok, const void* e
                                         const double* inv_freq, const float* w, float eps, int n_tok, int H, int V,
                                         float* h, void* a, cudaStream_t st) {
     if (H % 4 == 0 && H <= 8192 && (((uintptr_t)embed | (uintptr_t)w | (uintptr_t)h | (uintptr_t)a) & 15) == 0) {
-        const int wide = H / 4 < 512 ? (H / 4 + 31) / 32 * 32 : 512;
-        DISPATCH_T(dtype, return dk_launch(embed_position_rmsnorm_wide_kernel<T>, dim3(n_tok), dim3(wide), 0, st, tok, (const T*)embed, scale,
-                                           row_pos, inv_freq, w, eps, H, V, h, (T*)a));
+        // as many threads as the general kernel: a thread's squares are then the same ones
+        DISPATCH_T(dtype, return dk_launch(embed_position_rmsnorm_wide_kernel<T>, dim3(n_tok), dim3(row_threads(H)), H * sizeof(float), st, tok,
+                                           (const T*)embed, scale, row_pos, inv_freq, w, eps, H, V, h, (T*)a));
     }
     DISPATCH_T(dtype, return dk_launch(embed_position_rmsnorm_kernel<T>, dim3(n_tok), dim3(row_threads(H)), 0, st, tok,
                                        (const T*)embed, scale, row_pos, inv_freq, w, eps, H, V, h, (T*)a));

@@ -129,6 +129,26 @@ def test_embedding_with_a_position_vector(dtype, H, shift):
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("H", [4, 132, 516, 1024, 2560, 8192])
+def test_an_embedding_gives_the_same_bits_wherever_its_rows_lie(dtype, H):
+    """Table and weights on 16-byte boundaries (four columns a thread) and one number off them (a number at a time), with and without
+    positions: products, sines and the sum of squares are rounded alike."""
+    V, rows = 40, 129
+    table, weight = rnd(V * H, seed=16).to(dtype), 1 + 0.1 * rnd(H, seed=17)
+    tok = torch.randint(0, V, (rows,), generator=torch.Generator().manual_seed(18), dtype=torch.int32).to(DEV)
+    pos = torch.arange(rows, dtype=torch.int32, device=DEV) * 397 - 1
+    for inv in (10000.0 ** (-torch.arange(0, H, 2, device=DEV, dtype=torch.float64) / H), None):
+        got = []
+        for off in (0, 1):
+            embed = torch.empty(V * H + 8, dtype=dtype, device=DEV)[off:off + V * H].copy_(table).view(V, H)
+            w = torch.empty(H + 8, device=DEV)[off:off + H].copy_(weight)
+            h, a = torch.empty(rows, H, device=DEV), torch.empty(rows, H, dtype=dtype, device=DEV)
+            api.embed_position_rmsnorm(tok, embed, 1.3, pos, inv, w, 1e-6, h, a)
+            got.append((h.view(torch.int32), a.view(torch.int16 if dtype == torch.bfloat16 else torch.int32)))
+        assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("nkv,hd,hdv,extra,shift", [(8, 128, 128, 0, 0), (2, 64, 32, 8, 0), (3, 20, 12, 0, 0), (1, 128, 128, 3, 0),
                                                    (2, 64, 64, 0, 1), (1, 576, 0, 0, 0)])
 def test_keys_and_values_into_the_cache(dtype, nkv, hd, hdv, extra, shift):
