@@ -364,16 +364,14 @@ def decode_splits(n_seq, n_kv_heads, group, table_pages=0, max_splits=8, residen
     while a split keeps 16 pages (one sequence of 32,768 tokens in 8 splits of its 8 kv heads kept
     64 of 296 block slots busy: 0.55 of the copy peak for the step). Beyond that: enough for about
     six waves of blocks, which evens out sequences of unequal lengths (measured at batch 64: 133 us
-    unsplit, 115 us in four splits), of four pages at least where the table has fewer than 16 (64 sequences of 64 to 360 tokens, 8
-    pages: 16.5 us in one or two splits, 19.0 in four; of 20 to 60, one page: 8.9 in one, 12.4 in four)."""
+    unsplit, 115 us in four splits)."""
     if resident_blocks is None:
         resident_blocks = 2 * sm_count()
     blocks = n_seq * n_kv_heads * ((group + 15) // 16)
     if blocks <= resident_blocks:
         room = resident_blocks // blocks
         return max(1, min(max_splits, room), min(DECODE_MAX_SPLITS, room, table_pages // 16))
-    most = max_splits if not 0 < table_pages < 16 else max(1, min(max_splits, table_pages // 4))
-    return max(1, min(most, -(-6 * resident_blocks // blocks)))
+    return max(1, min(max_splits, -(-6 * resident_blocks // blocks)))
 
 
 def attention_decode_ws(n_seq, n_heads, head_dim, nsplit, device):

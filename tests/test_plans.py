@@ -76,15 +76,6 @@ def test_decode_splits_depend_on_the_batch_only_and_stay_within_what_the_merge_t
         assert api.decode_splits(1, 8, 4, 64) == 8 and api.decode_splits(1, 8, 4, 512) == 32 and api.decode_splits(8, 8, 4, 512) == 4
 
 
-def test_decode_splits_of_many_sequences_keep_four_pages_of_a_short_table():
-    for n_seq, nkv, group in itertools.product((40, 64, 500), (8, 16), (1, 4, 16)):
-        n = api.decode_splits(n_seq, nkv, group)
-        for pages in (1, 2, 4, 8, 16, 64):
-            got = api.decode_splits(n_seq, nkv, group, pages)
-            assert got == (n if pages >= 16 else max(1, min(n, pages // 4)))
-    assert api.decode_splits(8, 8, 4, 2) == api.decode_splits(8, 8, 4)      # all blocks at once: as before
-
-
 def test_gemm_tc_fills_gpu_is_about_the_last_wave():
     assert api.gemm_tc_fills_gpu(2048, 19456 // 2)            # 16 x 38 tiles: 4.1 waves
     assert not api.gemm_tc_fills_gpu(2048, 2560)              # 160 tiles on 148 SMs: a second wave of 12
