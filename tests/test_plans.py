@@ -76,6 +76,16 @@ def test_decode_splits_depend_on_the_batch_only_and_stay_within_what_the_merge_t
         assert api.decode_splits(1, 8, 4, 64) == 8 and api.decode_splits(1, 8, 4, 512) == 32 and api.decode_splits(8, 8, 4, 512) == 4
 
 
+def test_decode_splits_beyond_the_sms_do_not_hang_on_a_neighbours_length():
+    """More blocks than the SMs hold: a row's splits are those of the batch however many pages the longest sequence beside it has,
+    also in the masked kernel, whose windows see a few pages of any table."""
+    for n_seq, nkv, group in itertools.product((40, 64, 500), (8, 16), (1, 4, 16)):
+        n = api.decode_splits(n_seq, nkv, group)
+        for pages in (1, 2, 8, 15, 16, 17, 64):
+            assert api.decode_splits(n_seq, nkv, group, pages) == n
+            assert api.masked_decode_splits(n_seq, nkv, group, 64, 64 * pages, None) == min(n, pages + 2)
+
+
 def test_gemm_tc_fills_gpu_is_about_the_last_wave():
     assert api.gemm_tc_fills_gpu(2048, 19456 // 2)            # 16 x 38 tiles: 4.1 waves
     assert not api.gemm_tc_fills_gpu(2048, 2560)              # 160 tiles on 148 SMs: a second wave of 12
