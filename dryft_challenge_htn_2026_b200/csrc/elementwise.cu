@@ -273,7 +273,7 @@ __global__ void qk_norm_rope_write_kernel(const T* qkv, const float* parts, int 
 
 // The head's sum of squares in the order of qk_norm_rope_write_kernel, whose lane L holds the pairs L and (heads of 128) L + 32: here
 // pairs 4 l + c lie with lane l of each half of the head, c = 0..3. The 8 lanes of a quarter of the head (heads of 64: of a half) add
-// up one c (two); 10 shuffles with the caller's four instead of 24.
+// up one c (two): 6 (7) shuffles where four columns a lane one by one would take 20 (16).
 template <int HDT>
 __device__ __forceinline__ float head_squares(const float4& first, const float4& other, int lane) {
     const float t[4] = {pair_squares(first.x, other.x), pair_squares(first.y, other.y), pair_squares(first.z, other.z),
@@ -301,7 +301,8 @@ __device__ __forceinline__ float head_squares(const float4& first, const float4&
 // consecutive columns of a head and reads them as one float4 of every part, up to eight parts on their way at a time; the other half
 // of the rotation comes from the lane half a head further. Every sum, the squares' among them, is added up as above, so that a row's
 // result does not depend on where its tensors lie. Bound by the trip to the L2 after the wait. In a chain of its own, with
-// scalar loads before: 4 parts of one row of 48 heads of 128 3.6 -> 1.8 us, 9 parts of 64 rows 6.0 -> 3.1, 544 float32 rows 12.2 -> 10.9.
+// scalar loads before: 4 parts of one row of 48 heads of 128 2.3 -> 1.4 us, 9 parts of 64 rows 4.6 -> 3.0; 544 float32 rows 11.0 either
+// way. (64 registers: with the other half's norm weights kept instead of a second exchange 72, 2.8 us at 64 rows but 11.9 at 544.)
 template <typename T, int HDT>
 __global__ void qk_norm_rope_write_quad_kernel(const float* parts, int n_parts, size_t part_stride, float zero, T* q_out, T* dense_out,
                                                const float* __restrict__ qn, const float* __restrict__ kn,
@@ -318,7 +319,7 @@ __global__ void qk_norm_rope_write_quad_kernel(const float* parts, int n_parts, 
     const bool is_q = hidx < nh, is_v = hidx >= nh + nkv;
     const bool work = pos >= 0 && (is_q || write_kv || dense_out != nullptr);
     T* dst = nullptr;
-    float4 c = make_float4(1.f, 1.f, 1.f, 1.f), sn = make_float4(0.f, 0.f, 0.f, 0.f), w = c, wy = c;
+    float4 c = make_float4(1.f, 1.f, 1.f, 1.f), sn = make_float4(0.f, 0.f, 0.f, 0.f), w = c;
     const float* nw = is_v ? nullptr : is_q ? qn : kn;
     const bool turn = cos_t != nullptr && !is_v;
     if (work) {
@@ -334,7 +335,7 @@ __global__ void qk_norm_rope_write_quad_kernel(const float* parts, int n_parts, 
             c = *reinterpret_cast<const float4*>(cos_t + (size_t)pos * HALF + d % HALF);
             sn = *reinterpret_cast<const float4*>(sin_t + (size_t)pos * HALF + d % HALF);
         }
-        if (nw) w = *reinterpret_cast<const float4*>(nw + d), wy = *reinterpret_cast<const float4*>(nw + (d ^ HALF));
+        if (nw) w = *reinterpret_cast<const float4*>(nw + d);
     }
     pdl_launch_dependents();   // before the wait, as in qk_norm_rope_write_kernel
     pdl_wait();
@@ -351,16 +352,19 @@ __global__ void qk_norm_rope_write_quad_kernel(const float* parts, int n_parts, 
                 if (k + u < n_parts) x.x += v[u].x, x.y += v[u].y, x.z += v[u].z, x.w += v[u].w;
         }
     }
-    float4 y;                                                 // the same columns of the head's other half
-    y.x = __shfl_xor_sync(0xffffffffu, x.x, G / 2), y.y = __shfl_xor_sync(0xffffffffu, x.y, G / 2);
-    y.z = __shfl_xor_sync(0xffffffffu, x.z, G / 2), y.w = __shfl_xor_sync(0xffffffffu, x.w, G / 2);
     const bool second = d >= HALF;
+    // the same columns of the head's other half
+    auto other = [](const float4& a) {
+        return make_float4(__shfl_xor_sync(0xffffffffu, a.x, G / 2), __shfl_xor_sync(0xffffffffu, a.y, G / 2),
+                           __shfl_xor_sync(0xffffffffu, a.z, G / 2), __shfl_xor_sync(0xffffffffu, a.w, G / 2));
+    };
+    float4 y = other(x);
     const float ss = head_squares<HDT>(second ? y : x, second ? x : y, lane);
     if (nw) {
         const float rs = rsqrtf(ss / (float)HDT + eps);
         x.x = x.x * rs * w.x, x.y = x.y * rs * w.y, x.z = x.z * rs * w.z, x.w = x.w * rs * w.w;
-        y.x = y.x * rs * wy.x, y.y = y.y * rs * wy.y, y.z = y.z * rs * wy.z, y.w = y.w * rs * wy.w;
     }
+    y = other(x);
     if (!work) return;
     if (turn) {
         if (!second)
