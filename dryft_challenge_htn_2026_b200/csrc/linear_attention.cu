@@ -49,16 +49,15 @@ linear_attention_step_kernel(const T* q, const T* k, const T* v, long long ld, f
     const int r0 = cu_q ? cu_q[s] : s, r1 = cu_q ? cu_q[s + 1] : s + 1;
     const int tid = threadIdx.x, c = tid % cols_pad, rg = tid / cols_pad;
     const size_t ow = (size_t)nh * hdv;
-    const int pos0 = seq_pos0[s], slot = seq_slot[s];
     const float d = GATED ? 0.f : decay[h];
-    if (pos0 < 0) {
+    if (seq_pos0[s] < 0) {                               // its slot is not read: padding rows may lie behind the slots' end
         if (early) pdl_wait();
         pdl_launch_dependents();
         for (int t = r0; t < r1; t++)
             for (int i = tid; i < cols; i += LA_THREADS) out[(size_t)t * ow + (size_t)h * hdv + col0 + i] = 0.f;
         return;
     }
-    float* S = state + ((size_t)slot * nh + h) * (size_t)hd * hdv + col0;
+    float* S = state + ((size_t)seq_slot[s] * nh + h) * (size_t)hd * hdv + col0;
     float st[EPT];
 #pragma unroll
     for (int i = 0; i < EPT; i++) {
