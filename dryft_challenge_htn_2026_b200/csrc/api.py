@@ -41,8 +41,9 @@ _thread = _Thread()
 class dependent_launches:
     """``with dependent_launches():`` around the kernels of a model's step. Kernels launched here start under the end of the one
     before them, and some of them read before they wait for it: matrix products their weights, the norms and rotations their
-    weights, positions and tables, decode attention its positions, page ids and the cache pages before the newest token's. So
-    nothing launched in here may write any of those. The first launch on a stream waits for all that the stream held before, so
+    weights, positions and tables, decode attention its positions, page ids and the cache pages before the newest token's, single
+    tokens of a recurrence their positions, slots and decays (the states themselves behind the wait). So nothing launched in here may
+    write any of those. The first launch on a stream waits for all that the stream held before, so
     that the caller may have. Outside, where any call may read what the one before it wrote, every kernel is launched behind the full
     end of the one before. It holds for the calling thread only.
 

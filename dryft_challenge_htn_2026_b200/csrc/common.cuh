@@ -70,8 +70,10 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 // and fill their rings while the kernel before the short one is still at work. That is safe
 // because every kernel waits before it reads or writes anything that another kernel of the step
 // writes (a wait returns only when the kernel before has finished, which in turn has waited for
-// the one before it), and what a streaming kernel does before its wait reads only what no kernel
-// of the step writes: weights; positions, page ids and the cache pages of older tokens.
+// the one before it), and what a kernel does before its wait reads only what no kernel of the step
+// writes: weights and decays; positions, slots, page ids and the cache pages of older tokens. A
+// recurrent state is written by every token of it: it may be called into the L2 before the wait, but
+// is read behind it.
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;"); }
 
 // Cache policy for what a decode step reads exactly once (weights, the keys and values of a sequence):
