@@ -282,13 +282,15 @@ F32_DECODE_BYTES = 256 << 20        # most scratch memory for the pages' results
 F32_TILE_ROWS, F32_SHORT_TILE_ROWS = 64, 32  # rows (queries x the query heads of a kv head) a block of attention_prompt_f32 takes
 
 
-def f32_tile_rows(n_tok, n_heads, n_kv_heads):
-    """Rows a tile for a step of ``n_tok`` rows: while all tiles of 64 are on the SMs at once (two each) the step takes as long as its
-    longest tile, and tiles of 32 take two thirds of that a page. Us in tiles of 64 and 32, 32 heads of 128: 100 tokens 29 and 19,
-    300 63 and 54, 544 (272 tiles) 125 and 112; 700 and 300 (504 tiles) 169 and 206, eight of 150 (640 tiles) 83 and 88."""
-    group = n_heads // n_kv_heads
-    tiles = -(-n_tok // (F32_TILE_ROWS // group)) * n_kv_heads
-    return F32_SHORT_TILE_ROWS if tiles <= 2 * sm_count() else F32_TILE_ROWS
+def f32_prompt_us(tile_rows, longest, pages):
+    """How long attention_prompt_f32 takes, without its launch: ``longest`` pages of keys before the last rows of the tile that sees the
+    most, ``pages`` of all tiles and kv heads together. A page of 64 (32) rows takes a block alone on its SM 12.5 (8.2) us, two
+    blocks beside each other 18 (11.6); the blocks, two an SM, take tiles of all lengths, the longest first. Measured, 32 heads of 128,
+    us in tiles of 64 and 32: one sequence of 100 tokens 26 and 16, 300 61 and 52, 544 124 and 110; 700 and 300 167 and 204, nine of 64
+    24 and 26, eight of 150 82 and 87, 16 of 30 21 and 23, 30 of 17 35 and 28 (a second tile of 64 rows for one token), 64 of 5 30 and
+    20: the smaller of the two is taken in each."""
+    alone, shared = (12.5, 18.0) if tile_rows == F32_TILE_ROWS else (8.2, 11.6)
+    return max(alone * longest, shared * pages / (2 * sm_count()))
 
 
 def _need_f32_attention(q, out, k_store, v_store, page_table, n_heads, n_kv_heads, head_dim):

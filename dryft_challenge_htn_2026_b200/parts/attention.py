@@ -37,6 +37,38 @@ class QueryTiles(StepPlan):
         return np.stack([seq[order], q0[order]], 1).astype(np.int32).reshape(-1, 2)
 
 
+class F32QueryTiles(StepPlan):
+    """The same for float32 attention, in tiles of the height with the smaller modelled time (``api.f32_prompt_us``)."""
+
+    def __init__(self, n_heads, n_kv_heads, window):
+        self.n_kv_heads, self.group, self.window = n_kv_heads, n_heads // n_kv_heads, window or 0
+        self.key = ("query_tiles_f32", n_heads, n_kv_heads, self.window)
+
+    def plan(self, lens, pos0):
+        """(rows a tile, tiles)."""
+        lens, pos0 = np.asarray(lens, dtype=np.int64), np.asarray(pos0, dtype=np.int64)
+        best = None
+        for rows in (api.F32_TILE_ROWS, api.F32_SHORT_TILE_ROWS):
+            queries = rows // self.group
+            tiles = QueryTiles(queries).build(lens, pos0, False)
+            seq, q0 = tiles[:, 0], tiles[:, 1].astype(np.int64)
+            first = np.maximum(0, pos0[seq] + q0 - self.window + 1) // api.PAGE if self.window else 0
+            pages = (pos0[seq] + np.minimum(q0 + queries, lens[seq]) - 1) // api.PAGE - first + 1
+            us = api.f32_prompt_us(rows, int(pages.max()), int(pages.sum()) * self.n_kv_heads)
+            if best is None or us < best[0]:
+                best = us, (rows, tiles)
+        return best[1]
+
+    def build(self, lens, pos0, is_decode):
+        return QueryTiles(1).build(lens, pos0, True) if is_decode else self.plan(lens, pos0)[1]
+
+    def rows(self, ctx):
+        """Rows a tile of the list built for this step; worked out once a step."""
+        if self.key not in ctx.host:
+            ctx.host[self.key] = self.plan(ctx.host["lens"], ctx.host["pos0"])[0]
+        return ctx.host[self.key]
+
+
 class GQAAttention(Part):
     # how full the last wave of the tensor-core product's tiles must be for a prefill step's projection
     # to run as that product with norm, rotation and cache write in its epilogue (csrc.api.gemm_tc_qkv)
@@ -67,8 +99,7 @@ class GQAAttention(Part):
         self.paged_f32 = rt.dtype == torch.float32 and s.head_dim in api.F32_ATTENTION_HEAD_DIMS \
             and group <= api.F32_ATTENTION_MAX_GROUP
         self.tiles = QueryTiles(api.TC_TILE_ROWS if self.tc_prefill else api.MMA_TILE_ROWS) \
-            if rt.dtype == torch.bfloat16 else QueryTiles(api.F32_TILE_ROWS // group) if self.paged_f32 else None
-        self.short_tiles = QueryTiles(api.F32_SHORT_TILE_ROWS // group) if self.paged_f32 else None    # for short steps (api.f32_tile_rows)
+            if rt.dtype == torch.bfloat16 else F32QueryTiles(s.num_heads, s.num_kv_heads, s.window) if self.paged_f32 else None
 
     def param_decls(self):
         s = self.spec
@@ -94,7 +125,7 @@ class GQAAttention(Part):
         return [self.w_qkv, self.w_o]
 
     def step_plans(self):
-        return [t for t in (self.tiles, self.short_tiles) if t is not None]
+        return [self.tiles] if self.tiles is not None else []
 
     def cache_requests(self):
         s = self.spec
@@ -154,10 +185,8 @@ class GQAAttention(Part):
         if self.paged_f32 and ctx.is_decode:
             api.attention_decode_f32(q, o, kv.k, kv.v, ctx.row_pos, table, nh, nkv, hd, window, s.scale)
         elif self.paged_f32:
-            rows = api.f32_tile_rows(ctx.n_tok, nh, nkv)
-            tiles = self.tiles if rows == api.F32_TILE_ROWS else self.short_tiles
-            api.attention_prompt_f32(q, o, kv.k, kv.v, ctx.plans[tiles.key], ctx.cu_q, ctx.seq_pos0, table, nh, nkv, hd, window,
-                                     s.scale, rows)
+            api.attention_prompt_f32(q, o, kv.k, kv.v, ctx.plans[self.tiles.key], ctx.cu_q, ctx.seq_pos0, table, nh, nkv, hd, window,
+                                     s.scale, self.tiles.rows(ctx))
         elif dtype == torch.float32:
             api.attention_generic(q, o, kv.k, kv.v, ctx.row_pos, ctx.row_seq, table, nh, nkv, hd, window, s.scale)
         elif ctx.is_decode:

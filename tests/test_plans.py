@@ -3,7 +3,15 @@ splits decode attention gets. The kernels refuse plans that break these invarian
 must never produce one."""
 import itertools
 
+import pytest
+import torch
+
+from dryft_challenge_htn_2026_b200.cache import Cache
+from dryft_challenge_htn_2026_b200.config.specs import AttentionSpec
 from dryft_challenge_htn_2026_b200.csrc import api
+from dryft_challenge_htn_2026_b200.engine.batch import build_context
+from dryft_challenge_htn_2026_b200.parts import Runtime, build_part
+from dryft_challenge_htn_2026_b200.parts.attention import F32QueryTiles, QueryTiles
 
 
 def test_stream_plan_keeps_a_slice_of_x_in_shared_memory_and_splits_only_when_allowed():
@@ -84,6 +92,32 @@ def test_decode_splits_beyond_the_sms_do_not_hang_on_a_neighbours_length():
         for pages in (1, 2, 8, 15, 16, 17, 64):
             assert api.decode_splits(n_seq, nkv, group, pages) == n
             assert api.masked_decode_splits(n_seq, nkv, group, 64, 64 * pages, None) == min(n, pages + 2)
+
+
+@pytest.mark.parametrize("before,lens,rows", [(0, [544], 32), (0, [700, 300], 64), (0, [17] * 30, 32), (300, [17] * 30, 32), (0, [64] * 9, 64),
+                                              (0, [30] * 16, 64), (200, [30] * 20, 64), (0, [150] * 8, 64), (0, [5] * 64, 32), (0, [1, 2], 32)])
+def test_float32_attention_plans_one_list_of_tiles_by_the_pages_a_step_reads(before, lens, rows):
+    """Tiles end with their sequence, so that steps of as many tokens differ in their tiles; the heights measured as the faster
+    ones. The step uploads one list, and the kernel is told its height."""
+    nh, nkv = 32, 8
+    part = build_part(AttentionSpec(2560, nh, nkv, 128, 1.0), Runtime(torch.device("cpu"), torch.float32))
+    cache = Cache([part.cache_requests()], 64 * 300, 64, "cpu")
+    slots = [cache.begin() for _ in lens]
+    for s in slots:
+        cache.reserve(s, before), cache.commit(s, before)
+    ctx = build_context(cache, [(s, [0] * n, []) for s, n in zip(slots, lens)], torch.device("cpu"), plans=part.step_plans())
+    assert list(ctx.plans) == [part.tiles.key]
+    got = part.tiles.rows(ctx)
+    assert got == rows or api.sm_count() != 148
+    assert ctx.plans[part.tiles.key].tolist() == QueryTiles(got // 4).build(lens, [before] * len(lens), False).tolist()
+
+
+def test_float32_attention_of_layers_with_windows_has_lists_of_its_own():
+    tiles = F32QueryTiles(32, 8, 40)
+    assert tiles.key != F32QueryTiles(32, 8, None).key and tiles.build([1, 1], [3, 4], True).shape == (0, 2)
+    for lens, before in (([150] * 8, [4000] * 8), ([7, 70], [0, 63])):
+        rows, plan = tiles.plan(lens, before)
+        assert plan.tolist() == QueryTiles(rows // 4).build(lens, before, False).tolist()
 
 
 def test_gemm_tc_fills_gpu_is_about_the_last_wave():
