@@ -209,3 +209,30 @@ def test_recurrence_in_chunks_of_64_value_columns(lens):
     # scores and weights are bfloat16 operands of the products: 2^-8 of the terms' norm, states 2^-16
     assert float((out.double().view_as(want) - want).norm() / want.norm()) <= 2.0 ** -7
     assert float((state.double() - last).norm() / last.norm()) <= 2.0 ** -13
+
+
+@pytest.mark.parametrize("hdv", [64, 128])
+def test_value_columns_a_block_change_no_bit_of_the_recurrence(hdv):
+    """The same sequences together (blocks of 64 value columns), by halves (32) and one by one (16): outputs and states."""
+    nh, hd, lens = 16, 128, [64, 130, 1, 200, 63, 65, 300, 128] * (128 // hdv)
+    n, T = len(lens), sum(lens)
+    proj = rnd(T, 2 * nh * hd + nh * hdv, seed=19).to(torch.bfloat16)
+    decay = 1.0 - 2.0 ** -(2 + 4 * torch.arange(nh, device=DEV, dtype=torch.float32) / nh)
+    start, first = rnd(n, nh, hd, hdv, seed=20), [sum(lens[:i]) for i in range(n + 1)]
+
+    def run(at_once):
+        state, out = start.clone(), torch.full((T, nh * hdv), float("nan"), device=DEV)
+        for s in range(0, n, at_once):
+            e = min(n, s + at_once)
+            rows = proj[first[s]:first[e]].clone()            # q, k and v are overwritten by their activation
+            cu = torch.tensor([f - first[s] for f in first[s:e + 1]], dtype=torch.int32, device=DEV)
+            slot = torch.arange(s, e, dtype=torch.int32, device=DEV)
+            q, k, v = rows.split([nh * hd, nh * hd, nh * hdv], 1)
+            api.linear_attention_chunk_bf16(q, k, v, out[first[s]:first[e]], state, cu, slot, decay, e - s, nh, hd, hdv)
+        return out, state
+
+    want = run(n)
+    assert bool(want[0].isfinite().all())
+    for at_once in (n // 2, 1):
+        for a, b in zip(run(at_once), want):
+            assert torch.equal(a, b)
