@@ -139,8 +139,9 @@ def test_few_rows_give_the_bits_of_many(M, N, K):
 
 @pytest.mark.parametrize("nt", [16, 32, 48, 64, 96, 112])
 def test_groups_summed_in_tensor_memory_or_in_the_output(nt):
-    """A unit of several groups of K (the last one shorter): row tiles that leave tensor memory room for their sum (16, 48 to 96 rows)
-    and ones that do not, full and ragged, against the groups left in parts and added in order; xIELU on the finished sums only."""
+    """A unit of several groups of K (the last one shorter): row tiles whose buffers leave tensor memory room for their sum (of these 16,
+    48 and 96 rows) and ones that do not (32, 64, 112), full and ragged, against the groups left in parts and added in order. (Products
+    with an activation have one group.)"""
     M, N, K = 150, 200, 2884
     groups, length = api.f32_groups(N, K)
     assert groups > 2 and groups * length > (K + 63) // 64
