@@ -429,8 +429,10 @@ def sgemm(x, w, out, mode=MODE_STORE, act=(0.0, 0.0)):
     _check(lib, lib.dk_sgemm(_p(x), _p(w), _p(out), M, N, K, mode, c_float(act[0]), c_float(act[1]), _stream()), "sgemm")
 
 
-# inner size from which linear() takes gemm_f32_tc: sgemm takes 0.07 us a column of K however few the rows (12 us at 64, 17 at
-# 200, 71 at 1,028, launch included), gemm_f32_tc with its split of x 17 to 25 us at all of these
+# inner size from which linear() takes gemm_f32_tc; sgemm below it, with its own order of sums. Us of sgemm and of gemm_f32_tc with
+# its split of x in a graph, 2,560 outputs, at K = 64, 128, 256 and 1,028: 4 rows 5.5 and 4.5, 9.8 and 5.0, 18.3 and 6.0, 68.5 and 13.5;
+# 5 rows 5.5 and 5.8, 9.8 and 6.3, 18.3 and 7.4, 68.5 and 14.6; 300 rows 9.3 and 7.7, 16.1 and 8.4, 30.0 and 9.8, 106 and 20.8: by time
+# the line could lie at 128; it stays where it was, so that narrower products keep their bits
 F32_TC_MIN_K = 256
 F32_CHUNK = 64              # columns of K that gemm_f32_tc adds up in tensor memory at a time
 F32_MAX_ROW_TILE = 128      # rows of x a tile

@@ -12,10 +12,11 @@
 //   prompts: a block takes 64 or 32 rows (rows / G queries of one sequence x the G query heads of one kv head) through its pages. Q, K,
 //       V in shared memory (K's place takes P afterwards: 98 or 82 KB, two blocks an SM); S = Q.K^T with 4 x 4 (2 x 4) scores a
 //       thread, P.V with 4 (2) rows x HD / 16 columns a thread; keys that every row of the tile sees go four at a time, only the few
-//       behind them with a test a row. Bound by the chain load - scores - weights - P.V (9 us a page of 64 rows and SM with two
-//       blocks, of which the FMA pipe is busy 4.3; 5.8 a page of 32). The tiles with the most pages of all heads start first: with the
-//       tiles of one head after those of another the last head's longest tiles came last. 32 heads of 128: 100 tokens 33 -> 19 us,
-//       300 72 -> 54, 544 157 -> 112 (125 in tiles of 64), 1,000 394 -> 265, 4,000 3,970 -> 3,640.
+//       behind them with a test a row. Bound by the chain load - scores - weights - P.V, whose shared-memory reads the two blocks of
+//       an SM wait for: 18 us a page of 64 rows, 11.6 of 32, two blocks side by side (tiles of 32, 544 tokens: FMA pipe 37 %, issue
+//       slots 54 %, 2.5 of the 4 stalled warps an issue on shared memory). The tiles with the most pages of all heads start first:
+//       with the tiles of one head after those of another the last head's longest tiles came last. 32 heads of 128, that and tiles of
+//       64 -> now: 100 tokens 31 -> 16 us, 300 70 -> 53, 544 156 -> 110 (124 in tiles of 64), 1,000 397 -> 264, 4,000 3,970 -> 3,640.
 //   single tokens: a block a (sequence, kv head, page), the pages merged by a second kernel. 2 sequences of 100 tokens: 203 us with
 //       a warp a row, whose keys follow one another at 2 us each -> 7.2 + 2.3 us.
 #include "common.cuh"

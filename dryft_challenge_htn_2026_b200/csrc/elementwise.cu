@@ -752,7 +752,8 @@ __global__ void embed_position_rmsnorm_kernel(const int* tok, const T* __restric
 // The same for widths that are multiples of 4, up to 8,192, on 16-byte boundaries: a thread holds up to four fours of columns, and an
 // angle's sine and cosine are worked out together, once. The bits are those of the kernel above: product and sine are rounded apart,
 // and the squares, handed over in shared memory, are added up in its order (a row's start does not depend on where its tensors lie).
-// Bound by the sines and the float64 angles. (16,000 rows of 2,560, bfloat16: 195 us with every number's angle worked out by itself, now 119.)
+// Bound by its instructions (issue slots 60 % busy, float64 and special functions 3 and 16 % of their pipes) and the waits at its three
+// barriers: 16,000 rows of 2,560, bfloat16, 193 us with every number's angle worked out by itself, now 131; 8 rows 5.3 and 3.2.
 template <typename T>
 __global__ void __launch_bounds__(512)
 embed_position_rmsnorm_wide_kernel(const int* tok, const T* __restrict__ embed, float scale, const int* row_pos,

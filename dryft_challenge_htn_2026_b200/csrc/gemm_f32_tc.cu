@@ -33,10 +33,12 @@
 //               chunk (250 to 350 clocks together) run beside the mma of the other one's.
 //   x: FEW and at most 4 rows: the warp loads them as float32 and takes them apart itself, two chunks ahead; else TMA of the pieces
 //               ([3][M][Kp] bfloat16, made by split_rows before: as the B operand they come ready from shared memory).
-// Measured in a graph (2,560 wide layers of 9,728; one converting group, one mma warp, descriptors built at each mma and split_rows in
-// front of every product -> this kernel; sgemm before both): one row: q/k/v 16.4 -> 12.4 us, output projection 13.8 -> 9.6, gated
-// 60.9 -> 50.1, down 22.1 -> 18.0 (the weights' bytes take 9.6, 6.4, 30.5, 15.2), a head of 50,000 91 -> 82 (6.2 TB/s). 544 rows:
-// 118 -> 86, 112 -> 63, 354 -> 330, 166 -> 150 (of which the sums kept in tensor memory 99 -> 86, 71 -> 63, 156 -> 150).
+// Measured in a graph, dependent launches, weights not in the L2 (2,560 wide layers of 9,728; one converting group, one mma warp,
+// descriptors built at each mma and split_rows in front of every product -> this kernel). One row: q/k/v 14.9 -> 13.0 us, output
+// projection 12.0 -> 10.2, gated 57.8 -> 50.9, down 20.2 -> 18.6 (the weights' bytes take 9.6, 6.4, 30.5, 15.2), a head of 50,000
+// 87 -> 82 (6.2 TB/s). 544 rows: 113 -> 86, 100 -> 63, 362 -> 298, 167 -> 156 (the sums kept in tensor memory took 99 -> 86 and 71 -> 63
+// of that). The gated product's tensor pipe is 64 % busy at 544 rows; at one row 13 %, and its SMs 67 % of the time (203 units in two
+// waves).
 // Infinities, NaN and numbers beyond bfloat16's largest: a piece times a zero piece is NaN where the product is not. A
 // thread that finds a sum that is not finite works that one out again by plain FMA from x and W.
 #include <cuda.h>
